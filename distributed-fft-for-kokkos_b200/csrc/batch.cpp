@@ -50,7 +50,7 @@ Batch::Batch(std::vector<const Plan*> plans) : plans_(std::move(plans)) {
     if (p->is_rank_plan()) fail(kErrInvalidArgument, "batched execution needs plans over all ranks, not per-rank plans");
     for (bool fwd : {true, false})
       for (const Op& op : p->program(fwd))
-        if (op.type != Op::Stage)
+        if (op.type != Op::Stage || op.chirp)
           fail(kErrInvalidArgument, "batched execution needs fused plans whose stages are all FFT stage kernels");
   }
   dbl_ = plans_[0]->desc().dbl;

@@ -53,7 +53,8 @@ struct StageArgs {
   // dst.off, so the kernels select no table at run time)
   int64_t s_ta, s_tb, s_to0, s_to1, d_ta, d_tb, d_to0, d_to1;
   // register kernels: 1 = two complex64 lines per thread (fft_pair.cu), 2 =
-  // the same streaming tpc consecutive tiles along b per CTA
+  // the same streaming tpc consecutive tiles along b per CTA, 3 = TMA-fed, 4 =
+  // the two-pass kernel (fft_flex.cuh)
   int pairs;
   int tpc;
   // device error word of the plan: kernels with bounded waits set it when a
@@ -169,6 +170,32 @@ int batch_stage_lines(int n);
 // kind: kC2C, kR2C or kC2R (R2C / C2R: lines along a on both sides)
 cudaError_t launch_fft_batch(BatchParams& P, bool dbl, int kind, bool inverse, bool afast, cudaStream_t st);
 cudaError_t launch_fft_batch_pair(BatchParams& P, bool inverse, bool afast, cudaStream_t st);
+// Two-pass stage of lines of m = R1 R2 points (fft_flex.cuh), or the chirp-z
+// form of it (chirp != null: n-point lines through a convolution of length
+// m >= 2 n - 1); geometry, layouts and scale in the StageArgs.
+struct FlexArgs {
+  int n, m, R1, R2;
+  int swap;            // inverse C2C: real and imaginary parts swapped on load and store
+  int cls;             // register class: codelets up to 10, 16, 32 points
+  int B, lshift;       // complex lines per tile (two real lines each for R2C / C2R); log2 B of b-fast tiles
+  int nthreads;
+  int share;           // a-fast R2C / C2R: threads per line of the half-spectrum passes
+  unsigned magic1, magic2, magic_share;  // ceil(2^32 / R1), / R2, / share: exact divisions by multiply-high
+  int P0, P1;          // pitch of a line in the first / second exchange buffer
+  size_t smem;
+  const void* tw;      // [a < R2][b < R1] w_m^(a b), then [a < R1][b < R2]
+  const void* chirp;   // chirp-z: n values exp(-i pi (j^2 mod 2n) / n)
+  const void* filter;  // chirp-z: m values (see BlueArgs)
+};
+// R1 >= R2 with R1 R2 = m, both codelet lengths, as even as possible
+bool flex_split(int m, int* R1, int* R2);
+// convolution length of an n-point chirp-z line (0: none that splits)
+int flex_chirp_length(int n);
+// Fill F (all but the table pointers) for option opt of kFlexOptions: which
+// radix comes first, and lines per tile; false if the option does not exist.
+constexpr int kFlexOptions = 4;
+bool flex_config(bool dbl, int kind, bool afast, int n, int m, int opt, FlexArgs* F);
+cudaError_t launch_fft_flex(const StageArgs& A, const FlexArgs& F, bool dbl, int kind, bool inverse, cudaStream_t st);
 // Chirp-z (Bluestein) stage for line lengths the radix passes do not cover
 // (a prime factor above 13): X_k = c_k sum_j (x_j c_j) conj(c_{k-j}),
 // c_j = exp(-i pi j^2 / n) (conjugated for the inverse), as a circular

@@ -123,6 +123,34 @@ void host_fft(std::vector<long double>& re, std::vector<long double>& im) {
   }
 }
 
+// FFT of m long double values: radix 2 for powers of two, else the plain sum
+// over the m-th roots of unity (m is at most a few hundred points there).
+void host_dft(std::vector<long double>& re, std::vector<long double>& im) {
+  const std::size_t m = re.size();
+  if ((m & (m - 1)) == 0) {
+    host_fft(re, im);
+    return;
+  }
+  const long double pi = 3.141592653589793238462643383279502884L;
+  std::vector<long double> c(m), s(m), xr(re), xi(im);
+  for (std::size_t k = 0; k < m; ++k) {
+    const long double ang = -2.0L * pi * static_cast<long double>(k) / static_cast<long double>(m);
+    c[k] = cosl(ang);
+    s[k] = sinl(ang);
+  }
+  for (std::size_t k = 0; k < m; ++k) {
+    long double ar = 0.0L, ai = 0.0L;
+    for (std::size_t j = 0, e = 0; j < m; ++j) {
+      ar += xr[j] * c[e] - xi[j] * s[e];
+      ai += xr[j] * s[e] + xi[j] * c[e];
+      e += k;
+      if (e >= m) e -= m;
+    }
+    re[k] = ar;
+    im[k] = ai;
+  }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -166,6 +194,7 @@ Plan::Plan(const PlanDesc& d, bool on_device) : d_(d), on_device_(on_device) {
     if (d_err_) cudaFree(d_err_);
     for (auto& kv : blue_tables_)
       for (void* p : kv.second) cudaFree(p);
+    for (auto& kv : flex_tables_) cudaFree(kv.second);
     throw;
   }
 }
@@ -178,6 +207,7 @@ Plan::~Plan() {
   if (d_err_) cudaFree(d_err_);
   for (auto& kv : blue_tables_)
     for (void* p : kv.second) cudaFree(p);
+  for (auto& kv : flex_tables_) cudaFree(kv.second);
 }
 
 void Plan::analyze() {
@@ -343,6 +373,126 @@ const void* Plan::twiddle(std::size_t n) {
   return p;
 }
 
+// Twiddles of an m = r1 r2 point two-pass transform, w_m = exp(-2 pi i / m):
+// [a < r2][b < r1] w_m^(a b), then [a < r1][b < r2] (re, im interleaved).
+std::vector<double> two_pass_twiddles(int r1, int r2) {
+  const int m = r1 * r2;
+  const long double pi = 3.141592653589793238462643383279502884L;
+  std::vector<double> h;
+  h.reserve(4 * static_cast<std::size_t>(m));
+  auto put = [&](int a, int b) {
+    const long double ang = 2.0L * pi * static_cast<long double>(a * b) / static_cast<long double>(m);
+    h.push_back(static_cast<double>(cosl(ang)));
+    h.push_back(static_cast<double>(-sinl(ang)));
+  };
+  for (int a = 0; a < r2; ++a)
+    for (int b = 0; b < r1; ++b) put(a, b);
+  for (int a = 0; a < r1; ++a)
+    for (int b = 0; b < r2; ++b) put(a, b);
+  return h;
+}
+
+const void* Plan::flex_twiddle(int r1, int r2) {
+  auto key = std::make_pair(r1, r2);
+  auto it = flex_tables_.find(key);
+  if (it != flex_tables_.end()) return it->second;
+  const std::vector<double> h = two_pass_twiddles(r1, r2);
+  const std::vector<float> hf(h.begin(), h.end());
+  void* p = nullptr;
+  const std::size_t bytes = h.size() * (d_.dbl ? 8 : 4);
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    fail(kErrAlloc, "cudaMalloc of twiddle table failed");
+  }
+  flex_tables_[key] = p;
+  workspace_bytes_ += bytes;
+  cuda_check(cudaMemcpy(p, d_.dbl ? static_cast<const void*>(h.data()) : static_cast<const void*>(hf.data()), bytes,
+                        cudaMemcpyHostToDevice),
+             "twiddle upload");
+  return p;
+}
+
+void Plan::select_flex(Op& op, int opt) const {
+  const dev::FlexArgs& F = op.flex.at(opt);
+  op.flex_opt = opt;
+  dev::StageArgs& A = op.sa;
+  A.pairs = 4;
+  A.B = F.B;
+  const int per = op.kind == dev::kC2C ? F.B : 2 * F.B;
+  A.tiles_b = (A.Eb + per - 1) / per;
+  op.tiles = static_cast<unsigned>(static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1);
+}
+
+// The two-pass kernel's options of a stage whose geometry (axes, extents, row
+// orientation) is set: lengths that split into two codelets, or whose chirp-z
+// convolution does; rows of one orientation on both sides (R2C / C2R: along
+// a); every side addressable by line (separable tables, or general ones whose
+// rank blocks do not split a).  Fills op.flex and the line addressing; false
+// (op untouched) if the kernel does not take the stage.
+bool Plan::add_flex(Op& op) {
+  dev::StageArgs& A = op.sa;
+  const std::size_t a = static_cast<std::size_t>(A.a);
+  if (A.load_afast != A.store_afast || A.Eo0 > dev::fast_stage_max_grid_yz() ||
+      A.Eo1 > dev::fast_stage_max_grid_yz())
+    return false;
+  const int nh = A.n / 2 + 1;
+  if (A.na_in != (op.kind == dev::kC2R ? nh : A.n) || A.na_out != (op.kind == dev::kR2C ? nh : A.n)) return false;
+  struct Side {
+    int affine = 0, atab = 0;
+    std::int64_t base = 0, stride = 1;
+  } side[2];
+  for (int k = 0; k < 2; ++k) {
+    const int l = k == 0 ? op.src_layout : op.dst_layout;
+    const LayoutTables& T = tables_[l];
+    Side& s = side[k];
+    if (T.mode != 0) {
+      if (layouts_[l].topo[a] != 1) return false;
+      s.affine = 1;
+      continue;
+    }
+    const std::size_t len = layouts_[l].gext[a];
+    const std::int64_t* off = T.data.data() + T.off[a];
+    s.stride = len > 1 ? off[1] - off[0] : 1;
+    s.base = off[0];
+    for (std::size_t c = 1; c < len; ++c)
+      if (off[c] != off[0] + static_cast<std::int64_t>(c) * s.stride) s.atab = 1;
+    if (s.atab) {
+      s.base = 0;  // the table carries the whole offset along a
+      s.stride = 1;
+    }
+  }
+  int r1 = 0, r2 = 0;
+  const bool chirp = !radix_supported(static_cast<std::size_t>(A.n));
+  const int m = chirp ? dev::flex_chirp_length(A.n) : A.n;
+  if (m == 0 || !dev::flex_split(m, &r1, &r2)) return false;
+  std::vector<dev::FlexArgs> opts;
+  for (int o = 0; o < dev::kFlexOptions; ++o) {
+    dev::FlexArgs F;
+    if (!dev::flex_config(d_.dbl, op.kind, A.load_afast != 0, A.n, m, o, &F)) continue;
+    const int per = op.kind == dev::kC2C ? F.B : 2 * F.B;
+    if (static_cast<unsigned long long>((A.Eb + per - 1) / per) * A.Eo0 * A.Eo1 >= (1ull << 31)) continue;
+    opts.push_back(F);
+  }
+  if (opts.empty()) return false;
+  const void *ch = nullptr, *filt = nullptr, *finv = nullptr;
+  if (chirp) bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &ch, &filt, &finv);
+  for (auto& F : opts) {
+    F.tw = flex_twiddle(F.R1, F.R2);
+    F.chirp = ch;
+    F.filter = filt;
+  }
+  op.flex = opts;
+  A.src_line_affine = side[0].affine;
+  A.src_atab = side[0].atab;
+  A.src_abase = side[0].base;
+  A.src_astride = side[0].stride;
+  A.dst_line_affine = side[1].affine;
+  A.dst_atab = side[1].atab;
+  A.dst_abase = side[1].base;
+  A.dst_astride = side[1].stride;
+  return true;
+}
+
 // Chirp and filter tables of an n-point chirp-z stage with m-point FFTs, in
 // the plan's precision: chirp c_j = exp(-i pi (j^2 mod 2n) / n), j < n; the
 // forward filter is FFT_m(b) / m with b_j = conj(c_j) for j < n, b_{m-j} = b_j
@@ -379,7 +529,7 @@ void Plan::bluestein_tables(std::size_t n, std::size_t m, const void** chirp, co
           bi[m - j] = im;
         }
       }
-      host_fft(br, bi);
+      host_dft(br, bi);
       std::vector<long double> f(2 * m);
       for (std::size_t k = 0; k < m; ++k) {
         f[2 * k] = br[k] / static_cast<long double>(m);
@@ -541,6 +691,11 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
   A.scale = scale;
 
   if (!is_copy && !radix_supported(n)) {
+    op.chirp = true;
+    if (add_flex(op)) {
+      select_flex(op, 0);
+      return op;
+    }
     // chirp-z stage: a circular convolution of length m >= 2n - 1
     std::size_t m = 1;
     while (m < 2 * n - 1) m <<= 1;
@@ -728,6 +883,11 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
     const unsigned long long ft = static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1;
     if (ft >= (1ull << 31)) fail(kErrUnsupported, "too many tiles");
     op.tiles = static_cast<unsigned>(ft);
+    // the two-pass kernel as another variant for the tuner (it computes the
+    // same line addressing)
+    if (!A.comp) add_flex(op);
+  } else if (!is_copy && add_flex(op)) {
+    select_flex(op, 0);
   }
   return op;
 }
@@ -822,6 +982,7 @@ static cudaError_t launch_fast_op(const dev::StageArgs& A, bool dbl, int kind, b
 // TMA kernel needs a source the tensor map can address (16-byte aligned
 // pointer); the two-line b-fast kernels need 16-byte aligned buffers.
 cudaError_t Plan::launch_stage(const Op& op, dev::StageArgs A, cudaStream_t stream) const {
+  if (A.pairs == 4) return dev::launch_fft_flex(A, op.flex[op.flex_opt], d_.dbl, op.kind, op.inverse, stream);
   if (!op.fast) return dev::launch_fft_stage(A, d_.dbl, op.kind, op.inverse, op.nthreads, op.smem, op.tiles, stream);
   const bool misaligned = ((reinterpret_cast<std::uintptr_t>(A.in) | reinterpret_cast<std::uintptr_t>(A.out)) & 15) != 0;
   if (A.pairs == 3) {
@@ -1308,7 +1469,7 @@ void Plan::autotune() {
   load_tune_cache_locked();
   for (auto* progs : {&prog_[0], &prog_[1], &adj_[0], &adj_[1]}) {
     for (auto& op : *progs) {
-      if (op.type != Op::Stage || !op.fast) continue;
+      if (op.type != Op::Stage || (!op.fast && op.flex.empty())) continue;
       dev::StageArgs& A = op.sa;
 
       // Trial buffers: the op's own plan-owned buffers, else the scratch
@@ -1328,7 +1489,7 @@ void Plan::autotune() {
       const bool real = op.kind == dev::kR2C || op.kind == dev::kC2R;  // two real lines per register line
       const bool pair_ok = op.single_B != 0;                            // eligible for two lines per thread
       const bool tma_ok = op.tma.ok;                                    // eligible for the TMA-fed kernel
-      k << "fast:n" << A.n << (d_.dbl ? "f64" : "f32") << (op.inverse ? "i" : "f") << (A.load_afast ? "a" : "b")
+      k << (op.flex.empty() ? "fast:n" : op.fast ? "fast+flex:n" : "flex:n") << A.n << (d_.dbl ? "f64" : "f32") << (op.inverse ? "i" : "f") << (A.load_afast ? "a" : "b")
         << (op.kind == dev::kR2C ? "r2c" : op.kind == dev::kC2R ? "c2r" : "") << (pair_ok ? "P" : "")
         << (tma_ok ? "T" : "") << (A.comp ? "C" : "")
         << (A.src_line_affine || A.dst_line_affine || A.src_atab || A.dst_atab ? "G" : "") << ":" << A.Eb << "x"
@@ -1344,9 +1505,15 @@ void Plan::autotune() {
       const std::string key = k.str();
       // a configuration: lines per tile of the one-line kernel; kPairCode +
       // lines per tile of the two-line kernel; kStreamCode + tiles per CTA of
-      // its streaming variant; kTmaCode + lines per tile of the TMA-fed kernel
-      constexpr int kPairCode = 100000, kStreamCode = 200000, kTmaCode = 300000;
+      // its streaming variant; kTmaCode + lines per tile of the TMA-fed
+      // kernel; kFlexCode + option of the two-pass kernel
+      constexpr int kPairCode = 100000, kStreamCode = 200000, kTmaCode = 300000, kFlexCode = 400000;
+      const int nflex = static_cast<int>(op.flex.size());
       auto apply = [&](int code) {
+        if (code >= kFlexCode) {
+          select_flex(op, code - kFlexCode);
+          return;
+        }
         if (code >= kTmaCode) {
           A.pairs = 3;
           A.B = code - kTmaCode;
@@ -1362,7 +1529,10 @@ void Plan::autotune() {
         op.tiles = static_cast<unsigned>(static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1);
       };
       auto it = g_tune_cache.find(key);
-      if (it != g_tune_cache.end() && (it->second < kPairCode || pair_ok) && (it->second < kTmaCode || tma_ok)) {
+      if (it != g_tune_cache.end() &&
+          (it->second >= kFlexCode ? it->second - kFlexCode < nflex
+                                   : op.fast && (it->second < kPairCode || pair_ok) &&
+                                         (it->second < kTmaCode || tma_ok))) {
         apply(it->second);
         continue;
       }
@@ -1397,9 +1567,10 @@ void Plan::autotune() {
         for (int tpc : {4, 8, 16})
           if (tiles >= 2 * tpc) cand.push_back(kStreamCode + tpc);
       }
-      const int nopt = A.comp ? 0 : dev::fast_stage_line_options(d_.dbl, A.n, opts);
+      const int nopt = A.comp || !op.fast ? 0 : dev::fast_stage_line_options(d_.dbl, A.n, opts);
       for (int i = 0; i < nopt; ++i) cand.push_back(opts[i]);
-      int best = A.pairs == 3 ? kTmaCode + A.B : A.pairs == 2 ? kStreamCode + A.tpc : (A.pairs ? kPairCode : 0) + A.B;
+      for (int i = 0; i < nflex; ++i) cand.push_back(kFlexCode + i);
+      int best = A.pairs == 4 ? kFlexCode + op.flex_opt : A.pairs == 3 ? kTmaCode + A.B : A.pairs == 2 ? kStreamCode + A.tpc : (A.pairs ? kPairCode : 0) + A.B;
       float best_ms = std::numeric_limits<float>::max();
       cudaEvent_t e0, e1;
       cuda_check(cudaEventCreate(&e0), "tuner event");

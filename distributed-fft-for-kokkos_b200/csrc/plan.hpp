@@ -68,6 +68,9 @@ struct TmaSource {
 // the description (tma.cpp).
 bool tma_encode(void* map, const void* base, const TmaSource& t);
 
+// Twiddle tables of a two-pass transform (dev::FlexArgs::tw), re / im interleaved.
+std::vector<double> two_pass_twiddles(int r1, int r2);
+
 struct Op {
   enum Type { Stage, Pack, All2All, Unpack, Scale, Copy, Weight, BluePre, BlueMul, BluePost, FourTwiddle } type;
   int src = -1, dst = -1;  // buffer ids
@@ -80,10 +83,15 @@ struct Op {
                       // caller buffers turn out not to be 16-byte aligned
   int pair_B = 0;     // lines per tile of the two-line kernel, for TMA stages whose source
                       // cannot be described by a tensor map at run time
+  // two-pass kernel (fft_flex.cuh): its options (tile and radix order), the one
+  // in use; a register stage (fast) may run it too when the tuner picks it
+  std::vector<dev::FlexArgs> flex;
+  int flex_opt = 0;
   TmaSource tma;      // source description of a TMA-eligible b-fast pair stage
   // chirp-z stage (line length with a prime factor above 13): make_stage marks
   // it, push_stage expands it into pre / FFT / mul / inverse FFT / post ops
   bool blue = false;
+  bool chirp = false;  // the line length has no radix plan (chirp-z, in one kernel or several)
   int blue_m = 0;
   long long blue_lines = 0;
   const void* blue_chirp = nullptr;
@@ -135,6 +143,7 @@ class Plan {
   std::size_t launches(bool forward) const { return prog_[forward ? 0 : 1].size(); }
   std::size_t workspace_bytes() const { return workspace_bytes_; }
   bool on_device() const { return on_device_; }
+  double scale(bool forward) const { return forward ? scale_fwd_ : scale_bwd_; }
   // Device error word (0 or the code a kernel's bounded wait left); reset clears it.
   int device_error(bool reset) const;
   // Batched execution (batch.cpp): the fused program of a direction, the
@@ -209,6 +218,11 @@ class Plan {
   void push_stage(std::vector<Op>& prog, const Op& op);
   std::map<std::pair<std::size_t, std::size_t>, std::vector<void*>> blue_tables_;  // (n, m) -> chirp, filter fwd / inv
   void bluestein_tables(std::size_t n, std::size_t m, const void** chirp, const void** ffwd, const void** finv);
+  // Twiddles of an m = R1 R2 point two-pass stage (dev::FlexArgs::tw).
+  std::map<std::pair<int, int>, void*> flex_tables_;
+  const void* flex_twiddle(int r1, int r2);
+  void select_flex(Op& op, int opt) const;
+  bool add_flex(Op& op);
   std::int64_t add_geo(const Layout& L, const BlockInfo& b, std::size_t pc);
   void build_fused(bool forward);
   void build_literal(bool forward);
