@@ -4,8 +4,8 @@
 // four-step stages of lines too long for one stage.  The FFTs themselves are
 // ordinary register or generic stages on a plain (lines, m) array.
 // These kernels address the rank-blocked layouts element by element through
-// the layout tables: the path serves line lengths the radix passes cannot
-// (a prime factor above 13), not the hot shapes.
+// the layout tables: the path serves the chirp-z lines too long for one kernel
+// (fft_flex.cuh takes them up to about 512 points), not the hot shapes.
 #include "fft_stage.cuh"
 
 namespace dfft {

@@ -172,29 +172,23 @@ cudaError_t launch_fft_batch(BatchParams& P, bool dbl, int kind, bool inverse, b
 cudaError_t launch_fft_batch_pair(BatchParams& P, bool inverse, bool afast, cudaStream_t st);
 // Two-pass stage of lines of m = R1 R2 points (fft_flex.cuh), or the chirp-z
 // form of it (chirp != null: n-point lines through a convolution of length
-// m >= 2 n - 1); geometry, layouts and scale in the StageArgs.
+// m >= 2 n - 1); geometry, layouts, tile (A.B complex lines) and scale in the
+// StageArgs.
 struct FlexArgs {
-  int n, m, R1, R2;
-  int swap;            // inverse C2C: real and imaginary parts swapped on load and store
-  int cls;             // register class: codelets up to 10, 16, 32 points
-  int B, lshift;       // complex lines per tile (two real lines each for R2C / C2R); log2 B of b-fast tiles
-  int nthreads;
-  int share;           // a-fast R2C / C2R: threads per line of the half-spectrum passes
-  unsigned magic1, magic2, magic_share;  // ceil(2^32 / R1), / R2, / share: exact divisions by multiply-high
-  int P0, P1;          // pitch of a line in the first / second exchange buffer
-  size_t smem;
+  int n, m;
+  int inverse;         // set by the launcher
   const void* tw;      // [a < R2][b < R1] w_m^(a b), then [a < R1][b < R2]
   const void* chirp;   // chirp-z: n values exp(-i pi (j^2 mod 2n) / n)
-  const void* filter;  // chirp-z: m values (see BlueArgs)
+  const void* filter;  // chirp-z: m values (see BlueArgs), forward and inverse
+  const void* filter_inverse;
 };
-// R1 >= R2 with R1 R2 = m, both codelet lengths, as even as possible
-bool flex_split(int m, int* R1, int* R2);
-// convolution length of an n-point chirp-z line (0: none that splits)
+// whether the kernels take m-point lines (chirp: m-point convolutions), and
+// the split m = R1 R2, R1 >= R2
+bool flex_split(int m, bool chirp, int* R1, int* R2);
+// convolution length of an n-point chirp-z line (0: none long enough)
 int flex_chirp_length(int n);
-// Fill F (all but the table pointers) for option opt of kFlexOptions: which
-// radix comes first, and lines per tile; false if the option does not exist.
-constexpr int kFlexOptions = 4;
-bool flex_config(bool dbl, int kind, bool afast, int n, int m, int opt, FlexArgs* F);
+// complex lines per tile (two real lines each for R2C / C2R)
+int flex_lines(bool dbl, bool afast, int R1);
 cudaError_t launch_fft_flex(const StageArgs& A, const FlexArgs& F, bool dbl, int kind, bool inverse, cudaStream_t st);
 // Chirp-z (Bluestein) stage for line lengths the radix passes do not cover
 // (a prime factor above 13): X_k = c_k sum_j (x_j c_j) conj(c_{k-j}),

@@ -68,7 +68,8 @@ bool fast_stage_supported(int n) {
 
 cudaError_t launch_fft_fast(const StageArgs& A, bool dbl, bool inverse, bool afast, cudaStream_t st) {
   if (A.Eo0 > fast_stage_max_grid_yz() || A.Eo1 > fast_stage_max_grid_yz()) return cudaErrorInvalidValue;
-  if (general_stage(A)) return launch_fast_general(A, dbl, inverse, afast, st);
+  if (general_stage(A))
+    return dbl ? launch_fast_general_t<double>(A, inverse, afast, st) : launch_fast_general_t<float>(A, inverse, afast, st);
 #define DFFT_CASE(N_)                                                                 \
   case N_:                                                                            \
     return dbl ? launch_fast_t<double, N_>(A, inverse, afast, st)                     \
@@ -96,7 +97,7 @@ cudaError_t launch_fft_fast(const StageArgs& A, bool dbl, bool inverse, bool afa
 
 cudaError_t launch_fft_fast_real(const StageArgs& A, bool dbl, bool c2r, cudaStream_t st) {
   if (A.Eo0 > fast_stage_max_grid_yz() || A.Eo1 > fast_stage_max_grid_yz()) return cudaErrorInvalidValue;
-  if (general_stage(A)) return launch_real_general(A, dbl, c2r, st);
+  if (general_stage(A)) return dbl ? launch_real_general_t<double>(A, c2r, st) : launch_real_general_t<float>(A, c2r, st);
 #define DFFT_CASE(N_)                                                                          \
   case N_:                                                                                     \
     if (dbl) return c2r ? launch_real_n<double, N_, true>(A, st) : launch_real_n<double, N_, false>(A, st); \

@@ -86,8 +86,18 @@ inline cudaError_t launch_real_b(const StageArgs& A, cudaStream_t st) {
 // Launch of a general-layout stage (affine lines, axis-table sides or a
 // spectral pre-multiplier; fft_fast_general.cu): lines per tile A.B among
 // fast_lines, 1/2 and 1/4 of it.
-cudaError_t launch_fast_general(const StageArgs& A, bool dbl, bool inverse, bool afast, cudaStream_t st);
-cudaError_t launch_real_general(const StageArgs& A, bool dbl, bool c2r, cudaStream_t st);
+template <typename T>
+cudaError_t launch_fast_general_t(const StageArgs& A, bool inverse, bool afast, cudaStream_t st);
+template <typename T>
+cudaError_t launch_real_general_t(const StageArgs& A, bool c2r, cudaStream_t st);
+template <>
+cudaError_t launch_fast_general_t<float>(const StageArgs& A, bool inverse, bool afast, cudaStream_t st);
+template <>
+cudaError_t launch_fast_general_t<double>(const StageArgs& A, bool inverse, bool afast, cudaStream_t st);
+template <>
+cudaError_t launch_real_general_t<float>(const StageArgs& A, bool c2r, cudaStream_t st);
+template <>
+cudaError_t launch_real_general_t<double>(const StageArgs& A, bool c2r, cudaStream_t st);
 
 inline bool general_stage(const StageArgs& A) {
   return A.src_line_affine || A.dst_line_affine || A.src_atab || A.dst_atab || A.pre_mode;

@@ -2,7 +2,7 @@
 // (fft_fast.cuh): lines addressed as base + p * stride from the general layout
 // tables, exchange-buffer sides addressed through the axis table, and the
 // spectral pre-multiplier of the Navier-Stokes backward transforms.  A
-// translation unit of its own so that it compiles beside fft_fast.cu.
+// translation unit per precision (FAST_T, set by the build).
 #include "fft_fast.cuh"
 
 namespace dfft {
@@ -43,23 +43,22 @@ cudaError_t general_real_n(const StageArgs& A, cudaStream_t st) {
 #define DFFT_GENERAL_LENGTHS(X) \
   X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096) X(24) X(48) X(96) X(192) X(384) X(768)
 
-cudaError_t launch_fast_general(const StageArgs& A, bool dbl, bool inverse, bool afast, cudaStream_t st) {
+template <>
+cudaError_t launch_fast_general_t<FAST_T>(const StageArgs& A, bool inverse, bool afast, cudaStream_t st) {
   switch (A.n) {
 #define DFFT_CASE(N_) \
-  case N_:            \
-    return dbl ? general_fast_t<double, N_>(A, inverse, afast, st) : general_fast_t<float, N_>(A, inverse, afast, st);
+  case N_: return general_fast_t<FAST_T, N_>(A, inverse, afast, st);
     DFFT_GENERAL_LENGTHS(DFFT_CASE)
 #undef DFFT_CASE
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_real_general(const StageArgs& A, bool dbl, bool c2r, cudaStream_t st) {
+template <>
+cudaError_t launch_real_general_t<FAST_T>(const StageArgs& A, bool c2r, cudaStream_t st) {
   switch (A.n) {
-#define DFFT_CASE(N_)                                                                                          \
-  case N_:                                                                                                     \
-    if (dbl) return c2r ? general_real_n<double, N_, true>(A, st) : general_real_n<double, N_, false>(A, st); \
-    return c2r ? general_real_n<float, N_, true>(A, st) : general_real_n<float, N_, false>(A, st);
+#define DFFT_CASE(N_) \
+  case N_: return c2r ? general_real_n<FAST_T, N_, true>(A, st) : general_real_n<FAST_T, N_, false>(A, st);
     DFFT_GENERAL_LENGTHS(DFFT_CASE)
 #undef DFFT_CASE
     default: return cudaErrorInvalidValue;

@@ -1,8 +1,10 @@
-// Host side of the two-pass stage (fft_flex.cuh): which lengths it takes, its
-// tiles, and the launch.
+// Host side of the two-pass stage (fft_flex.cuh): which lengths it takes, and
+// the launch.
 #include <algorithm>
+#include <map>
 
 #include "fft_flex.cuh"
+#include "fft_flex_lengths.h"
 
 namespace dfft {
 namespace dev {
@@ -11,125 +13,78 @@ using namespace flex;
 
 namespace {
 
-#define DFFT_OK(R_) case R_:
-bool small_codelet(int r) {
-  switch (r) {
-    DFFT_FLEX_R1(DFFT_OK) return true;
-    default: return false;
-  }
-}
-bool large_codelet(int r) {
-  switch (r) {
-    DFFT_FLEX_R2(DFFT_OK) return true;
-    default: return false;
-  }
-}
-#undef DFFT_OK
-// both radices in one register class's kernels
-bool codelet_pair(int a, int b) { return (small_codelet(a) && small_codelet(b)) || (large_codelet(a) && large_codelet(b)); }
+struct Split {
+  int m, r1, r2;
+};
+#define DFFT_SPLIT(M_, R1_, R2_) {M_, R1_, R2_},
+const Split kPlain[] = {DFFT_FLEX_PLAIN_0(DFFT_SPLIT) DFFT_FLEX_PLAIN_1(DFFT_SPLIT) DFFT_FLEX_PLAIN_2(DFFT_SPLIT)
+                            DFFT_FLEX_PLAIN_3(DFFT_SPLIT) DFFT_FLEX_PLAIN_4(DFFT_SPLIT) DFFT_FLEX_PLAIN_5(DFFT_SPLIT)
+                                DFFT_FLEX_PLAIN_6(DFFT_SPLIT) DFFT_FLEX_PLAIN_7(DFFT_SPLIT)};
+const Split kChirp[] = {DFFT_FLEX_CHIRP_0(DFFT_SPLIT) DFFT_FLEX_CHIRP_1(DFFT_SPLIT) DFFT_FLEX_CHIRP_2(DFFT_SPLIT)
+                            DFFT_FLEX_CHIRP_3(DFFT_SPLIT)};
+#undef DFFT_SPLIT
 
-unsigned magic(int d) { return static_cast<unsigned>(((1ull << 32) + d - 1) / d); }
+template <typename T, bool CHIRP, int... G>
+std::map<int, Entry> all_entries() {
+  std::map<int, Entry> all;
+  auto add = [&](const Entry* (*get)(int*)) {
+    int n = 0;
+    const Entry* e = get(&n);
+    for (int i = 0; i < n; ++i) all[e[i].m] = e[i];
+  };
+  (add(&Group<T, CHIRP, G>::entries), ...);
+  return all;
+}
+
+const Entry* find_entry(bool dbl, bool chirp, int m) {
+  static const std::map<int, Entry> tables[4] = {
+      all_entries<float, false, 0, 1, 2, 3, 4, 5, 6, 7>(), all_entries<float, true, 0, 1, 2, 3>(),
+      all_entries<double, false, 0, 1, 2, 3, 4, 5, 6, 7>(), all_entries<double, true, 0, 1, 2, 3>()};
+  const auto& t = tables[(dbl ? 2 : 0) + (chirp ? 1 : 0)];
+  const auto it = t.find(m);
+  return it == t.end() ? nullptr : &it->second;
+}
 
 }  // namespace
 
-// The most even split: the kernel's registers (and so its resident threads)
-// follow the larger codelet.
-bool flex_split(int m, int* R1, int* R2) {
-  int best = 0;
-  for (int r2 = 2; r2 * r2 <= m; ++r2)
-    if (m % r2 == 0 && codelet_pair(m / r2, r2)) best = r2;
-  if (best == 0) return false;
-  *R1 = m / best;
-  *R2 = best;
-  return true;
+bool flex_split(int m, bool chirp, int* R1, int* R2) {
+  auto find = [&](const Split* s, const Split* end) {
+    const Split* f = std::find_if(s, end, [&](const Split& x) { return x.m == m; });
+    if (f == end) return false;
+    *R1 = f->r1;
+    *R2 = f->r2;
+    return true;
+  };
+  return chirp ? find(std::begin(kChirp), std::end(kChirp)) : find(std::begin(kPlain), std::end(kPlain));
 }
 
-// The smallest m >= 2n - 1 that splits into codelets without a factor 11 or
-// 13 (those codelets cost O(R^2) operations).
 int flex_chirp_length(int n) {
-  for (int m = 2 * n - 1; m <= 32 * 32; ++m) {
-    int r1 = 0, r2 = 0;
-    if (m % 11 != 0 && m % 13 != 0 && flex_split(m, &r1, &r2)) return m;
-  }
-  return 0;
+  int best = 0;
+  for (const Split& s : kChirp)
+    if (s.m >= 2 * n - 1 && (best == 0 || s.m < best)) best = s.m;
+  return best;
 }
 
-// Options: bit 0 swaps the radices (a-fast rows are read in runs of R2 and
-// written in runs of R1 elements), bit 1 halves the tile.  Tiles: a-fast about
-// 256 complex64 or 192 complex128 butterflies; b-fast rows of 128 bytes.
-bool flex_config(bool dbl, int kind, bool afast, int n, int m, int opt, FlexArgs* F) {
-  if (kind != kC2C && !afast) return false;
-  if (opt < 0 || opt >= kFlexOptions) return false;
-  const bool chirp = m != n;
-  int r1 = 0, r2 = 0;
-  if (!flex_split(m, &r1, &r2)) return false;
-  if ((opt & 1) && r1 == r2) return false;
-  *F = FlexArgs{};
-  F->n = n;
-  F->m = m;
-  F->R1 = (opt & 1) ? r2 : r1;
-  F->R2 = (opt & 1) ? r1 : r2;
-  F->cls = r1 <= 10 ? 0 : r1 <= 16 ? 1 : 2;
-  const size_t ce = dbl ? 16 : 8;
-  const int odd1 = F->R1 | 1, odd2 = F->R2 | 1;
-  F->P0 = afast ? F->R2 * odd1 : m;
-  F->P1 = chirp ? (afast ? F->R1 * odd2 : m) : 0;
-  const int zn = afast ? (n | 1) : n;
-  if (kind == kC2R || (kind == kR2C && !chirp)) F->P1 = std::max(F->P1, zn);
-  if (kind == kR2C && chirp) F->P0 = std::max(F->P0, zn);
-  const int most = std::max(F->R1, F->R2);
-  int B = afast ? std::max(1, (dbl ? 192 : 256) / most) : (dbl ? 8 : 16);
-  if (opt & 2) {
-    if (B < 2) return false;
-    B /= 2;
-  }
-  const size_t line = (static_cast<size_t>(F->P0) + F->P1) * ce;
-  while (B > 1 && line * B > 100 * 1024) B /= 2;
-  if (line * B > 227 * 1024) return false;
-  F->B = B;
-  F->smem = line * B;
-  if (!afast)
-    while ((1 << F->lshift) < B) ++F->lshift;
-  const int total = B * most, cap = dbl ? 256 : 512;
-  const int loops = (total + cap - 1) / cap;
-  F->nthreads = std::min(cap, ((total + loops - 1) / loops + 31) / 32 * 32);
-  F->share = F->nthreads / B;
-  if (F->share < 2) return false;
-  F->magic1 = magic(F->R1);
-  F->magic2 = magic(F->R2);
-  F->magic_share = magic(F->share);
-  return true;
+int flex_lines(bool dbl, bool afast, int R1) {
+  return dbl ? tile_lines<double>(afast, R1) : tile_lines<float>(afast, R1);
 }
-
-namespace flex {
-#define DFFT_DECL(T, CLS, CHIRP) \
-  template <>                    \
-  cudaError_t launch_class<T, CLS, CHIRP>(const StageArgs& A, const FlexArgs& F, int kind, cudaStream_t st);
-DFFT_DECL(float, 0, false) DFFT_DECL(float, 1, false) DFFT_DECL(float, 2, false)
-DFFT_DECL(float, 0, true) DFFT_DECL(float, 1, true) DFFT_DECL(float, 2, true)
-DFFT_DECL(double, 0, false) DFFT_DECL(double, 1, false) DFFT_DECL(double, 2, false)
-DFFT_DECL(double, 0, true) DFFT_DECL(double, 1, true) DFFT_DECL(double, 2, true)
-#undef DFFT_DECL
-
-template <typename T, bool CHIRP>
-static cudaError_t launch_any_class(const StageArgs& A, const FlexArgs& F, int kind, cudaStream_t st) {
-  switch (F.cls) {
-    case 0: return launch_class<T, 0, CHIRP>(A, F, kind, st);
-    case 1: return launch_class<T, 1, CHIRP>(A, F, kind, st);
-    case 2: return launch_class<T, 2, CHIRP>(A, F, kind, st);
-    default: return cudaErrorInvalidValue;
-  }
-}
-}  // namespace flex
 
 cudaError_t launch_fft_flex(const StageArgs& A, const FlexArgs& F0, bool dbl, int kind, bool inverse,
                             cudaStream_t st) {
   if (A.Eo0 > fast_stage_max_grid_yz() || A.Eo1 > fast_stage_max_grid_yz()) return cudaErrorInvalidValue;
+  const Entry* e = find_entry(dbl, F0.chirp != nullptr, F0.m);
+  if (!e) return cudaErrorInvalidValue;
   FlexArgs F = F0;
-  F.swap = (kind == kC2C && inverse) ? 1 : 0;
-  if (F.chirp)
-    return dbl ? launch_any_class<double, true>(A, F, kind, st) : launch_any_class<float, true>(A, F, kind, st);
-  return dbl ? launch_any_class<double, false>(A, F, kind, st) : launch_any_class<float, false>(A, F, kind, st);
+  F.inverse = inverse ? 1 : 0;
+  const bool af = A.load_afast != 0;
+  LaunchFn fn = nullptr;
+  if (kind == kC2C)
+    fn = af ? e->c2c_a : e->c2c_b;
+  else if (kind == kR2C && af)
+    fn = e->r2c;
+  else if (kind == kC2R && af)
+    fn = e->c2r;
+  return fn ? fn(A, F, st) : cudaErrorInvalidValue;
 }
 
 }  // namespace dev

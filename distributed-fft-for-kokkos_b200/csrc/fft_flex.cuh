@@ -1,29 +1,39 @@
-// Two-pass FFT stage for lines of m = R1 R2 points, R1 and R2 any two codelet
-// lengths up to 32 (sm_100a): every 2^a 3^b 5^c 7^d 11^e 13^f length up to
-// about 700 that splits so, and, through the chirp-z convolution, every other
-// length n whose 2 n - 1 fits such an m.
+// Two-pass FFT stage for lines of m = R1 R2 points, R1 >= R2 two codelet
+// lengths up to 32 (sm_100a): the 2^a 3^b 5^c 7^d lengths up to 512 that split
+// so (and some up to 1024, and short multiples of 11 and 13), and, through the
+// chirp-z convolution, every other length n whose 2 n - 1 fits such an m.
 //
 // What bounds it: bytes.  A tile of B lines is read from global memory once
 // and written once; between the two passes a line crosses shared memory once
-// (chirp-z: twice).  Pass 1 gives every thread an R1-point codelet whose inputs
-// it loads itself, R1 independent loads in flight per thread; it leaves row j
-// of the line's R2 x R1 matrix in shared memory; pass 2 reads columns, applies
-// the twiddle w_m^(j r) and stores straight to global memory.  So there is one
-// barrier between loads and stores, and the CTAs of an SM, each at a different
-// point, keep the memory busy.
+// (chirp-z: twice).  Pass 1 gives every thread one R1-point codelet whose
+// inputs it loads itself, R1 independent loads in flight; it leaves row j of
+// the line's R2 x R1 matrix in shared memory; pass 2 reads columns, applies
+// the twiddle w_m^(j r) and stores straight to global memory.
 //
-// Measured (B200, forward + backward transform, before: the table-driven
-// shared-memory kernel of fft_stage.cu, chirp-z as five launches): 300 x 250 x
-// 360 complex64 3816 -> 810 us, 200 x 180 x 252 R2C / C2R double 1633 -> 467 us,
-// 131 x 105 x 157 R2C / C2R double 768 -> 331 us.
+// Measured (B200, forward + backward; before: the table-driven kernel of
+// fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
+// kernels): 300 x 250 x 360 complex64 3818 -> 593 us, 200 x 180 x 252 R2C / C2R
+// double 1633 -> 213 us, 131 x 105 x 157 R2C / C2R double 766 -> 187 us, 256^3
+// complex128 644 -> 558 us, 384^3 R2C / C2R double 1568 -> 1158 us.  On 2^k and
+// 3 2^k lines the tuner chooses between this kernel and the older ones, which
+// stay ahead on complex64 (two lines per thread) and short stages.
 //
-// The radices are run-time values (a switch over compile-time codelets), one
-// kernel per register class: codelets up to 10, 16 and 32 points.
+// The radices are template arguments, a kernel per length: with run-time
+// radices (a switch over codelets in one kernel: 810, 467, 331, 608 us and no
+// gain above) the registers were those of the largest codelet and every
+// shared-memory and global offset was computed, 90 instructions a point at
+// 10-20 % occupancy.  Here offsets are immediates and the registers follow R1.
+// CTAs are small (about 128 threads, one
+// butterfly each per pass), so that an SM holds many, each at a different
+// point between its loads and stores.
 //
 // Thread mapping: a-fast rows (unit stride along the FFT axis) take the
 // butterflies of a line on consecutive threads, with the matrix rows padded
 // to an odd pitch; b-fast rows (unit stride along the tile axis) take the B
-// lines of a tile on consecutive threads.
+// lines of a tile on consecutive threads, 128-byte rows.
+//
+// Inverse transforms take the forward codelets' outputs in reverse order,
+// X_{m-k}.
 #pragma once
 
 #include "fft_codelet.cuh"
@@ -34,49 +44,61 @@ namespace flex {
 
 using codelet::Dft;
 
-template <typename T, int CLS>
-struct Bounds {
-  // complex64: 512 threads (128 registers); complex128: 256 threads, two CTAs
-  // (128 registers) up to 16-point codelets, one (255 registers) above
-  static constexpr bool f32 = sizeof(T) == 4;
-  static constexpr int threads = f32 ? 512 : 256;
-  static constexpr int blocks = f32 ? 1 : (CLS < 2 ? 2 : 1);
+// Resident threads per SM the registers are sized for: what the R1 values of a
+// thread, its addresses and the codelet's temporaries take without spilling
+// (more for C2R lines, which load both half spectra, and for the chirp-z form).
+template <typename T>
+constexpr int resident_threads(int r, bool more) {
+  if (sizeof(T) == 4)
+    return more ? (r <= 12 ? 896 : r <= 16 ? 768 : r <= 21 ? 576 : 512)
+                : (r <= 8 ? 1280 : r <= 12 ? 1024 : r <= 16 ? 896 : r <= 21 ? 640 : r <= 25 ? 576 : 512);
+  return more ? (r <= 8 ? 768 : r <= 10 ? 640 : r <= 12 ? 512 : r <= 16 ? 448 : r <= 21 ? 320 : r <= 25 ? 288 : 256)
+              : (r <= 8 ? 896 : r <= 10 ? 768 : r <= 12 ? 640 : r <= 16 ? 512 : r <= 21 ? 448 : r <= 25 ? 384 : 256);
+}
+
+// Lines per tile: b-fast rows of at least 128 bytes; about 128 threads.
+template <typename T>
+constexpr int tile_lines(bool afast, int r) {
+  if (afast) return 128 / r > 1 ? 128 / r : 1;
+  int b = sizeof(T) == 4 ? 16 : 8;
+  while (b * r < 64) b *= 2;
+  return b;
+}
+
+template <typename T, int KIND, bool AFAST, int R1, int R2, bool CHIRP>
+struct Shape {
+  static constexpr int B = tile_lines<T>(AFAST, R1);
+  static constexpr int NT = (B * R1 + 31) / 32 * 32;
+  // a line's elements in shared memory: the R2 x R1 matrix (chirp-z: also the
+  // R1 x R2 one of the way back), or the line in natural order
+  static constexpr int m = R1 * R2, odd1 = R1 | 1, odd2 = R2 | 1;
+  static constexpr int p1 = R2 * odd1, p2 = CHIRP ? R1 * odd2 : 0, pn = m | 1;
+  static constexpr int P = AFAST ? (p1 > p2 ? (p1 > pn ? p1 : pn) : (p2 > pn ? p2 : pn)) : m;
+  static constexpr size_t smem = sizeof(cplx<T>) * B * P;
+  static constexpr int fit = resident_threads<T>(R1, CHIRP || KIND == kC2R) / NT;
+  static constexpr int blocks = fit > 0 ? fit : 1;
 };
 
 // positions of a line: affine, or from the axis table
 struct Line {
-  int64_t base, stride;
+  int64_t base;
+  int stride;
   const int64_t* tab;
-  __device__ __forceinline__ int64_t at(int p) const { return base + (tab ? __ldg(tab + p) : p * stride); }
 };
-
-// f(r, offset of position p0 + r * step) for r < R with p0 + r * step < lim
-// (LIM: else every r); one affine or one table loop, no choice per element
-template <int R, bool LIM, typename Fn>
-__device__ __forceinline__ void each(const Line& l, int p0, int step, int lim, Fn&& f) {
-  if (l.tab) {
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (!LIM || p0 + r * step < lim) f(r, l.base + __ldg(l.tab + p0 + r * step));
-  } else {
-    const int64_t b = l.base + p0 * l.stride, st = step * l.stride;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (!LIM || p0 + r * step < lim) f(r, b + r * st);
-  }
-}
 
 __device__ __forceinline__ Line src_line(const StageArgs& A, int lb, int co0, int co1) {
   Line l;
   l.tab = nullptr;
   if (A.src_line_affine) {
-    radix::line_affine(A.src, A, lb, co0, co1, &l.base, &l.stride);
+    int64_t s;
+    radix::line_affine(A.src, A, lb, co0, co1, &l.base, &s);
+    l.stride = static_cast<int>(s);
     return l;
   }
   l.base = A.src_abase + __ldg(A.src.t + A.s_tb + lb);
   if (A.o0 >= 0) l.base += __ldg(A.src.t + A.s_to0 + co0);
   if (A.o1 >= 0) l.base += __ldg(A.src.t + A.s_to1 + co1);
-  l.stride = A.src_astride;
+  l.stride = static_cast<int>(A.src_astride);
   if (A.src_atab) l.tab = A.src.t + A.s_ta;
   return l;
 }
@@ -85,316 +107,310 @@ __device__ __forceinline__ Line dst_line(const StageArgs& A, int lb, int co0, in
   Line l;
   l.tab = nullptr;
   if (A.dst_line_affine) {
-    radix::line_affine(A.dst, A, lb, co0, co1, &l.base, &l.stride);
+    int64_t s;
+    radix::line_affine(A.dst, A, lb, co0, co1, &l.base, &s);
+    l.stride = static_cast<int>(s);
     return l;
   }
   l.base = A.dst_abase + __ldg(A.dst.t + A.d_tb + lb);
   if (A.o0 >= 0) l.base += __ldg(A.dst.t + A.d_to0 + co0);
   if (A.o1 >= 0) l.base += __ldg(A.dst.t + A.d_to1 + co1);
-  l.stride = A.dst_astride;
+  l.stride = static_cast<int>(A.dst_astride);
   if (A.dst_atab) l.tab = A.dst.t + A.d_ta;
   return l;
 }
 
-template <typename T, int KIND, bool AFAST, bool CHIRP>
-struct Tile {
+// f(r, offset of position p0 + r * STEP of the line) for r < R; LIM: only
+// positions below lim.  a-fast lines have unit stride.
+template <int R, int STEP, bool AFAST, bool LIM, typename Fn>
+__device__ __forceinline__ void positions(const Line& l, int p0, int lim, Fn&& f) {
+  if (l.tab) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!LIM || p0 + r * STEP < lim) f(r, l.base + __ldg(l.tab + p0 + r * STEP));
+  } else if (AFAST) {
+    const int64_t b = l.base + p0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!LIM || p0 + r * STEP < lim) f(r, b + r * STEP);
+  } else {
+    // (len - 1) * stride < 2^31 (host check)
+    const int64_t b = l.base + static_cast<int64_t>(p0) * l.stride;
+    const int st = STEP * l.stride;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (!LIM || p0 + r * STEP < lim) f(r, b + r * st);
+  }
+}
+
+// The same for outputs k = j + r * STEP of an m-point transform, m - k for
+// inverse ones (position 0 stays).
+template <int R, int STEP, int M, bool AFAST, typename Fn>
+__device__ __forceinline__ void outputs(const Line& l, int j, bool inverse, Fn&& f) {
+  if (!inverse) {
+    positions<R, STEP, AFAST, false>(l, j, 0, f);
+    return;
+  }
+  const int p0 = j == 0 ? 0 : M - j;
+  if (l.tab) {
+    f(0, l.base + __ldg(l.tab + p0));
+#pragma unroll
+    for (int r = 1; r < R; ++r) f(r, l.base + __ldg(l.tab + M - j - r * STEP));
+  } else if (AFAST) {
+    f(0, l.base + p0);
+    const int64_t b = l.base + M - j;
+#pragma unroll
+    for (int r = 1; r < R; ++r) f(r, b - r * STEP);
+  } else {
+    f(0, l.base + static_cast<int64_t>(p0) * l.stride);
+    const int64_t b = l.base + static_cast<int64_t>(M - j) * l.stride;
+    const int st = STEP * l.stride;
+#pragma unroll
+    for (int r = 1; r < R; ++r) f(r, b - r * st);
+  }
+}
+
+// Column j of the matrix of R1 wide rows: R values, twiddled (tw [r][j] = w^(j r)).
+template <typename T, int R, int R1, int PITCH>
+__device__ __forceinline__ void load_column(const cplx<T>* s, const cplx<T>* tw, int j, cplx<T>* v) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = s[r * PITCH];
+#pragma unroll
+  for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(tw + r * R1 + j));
+}
+
+template <typename T, int KIND, bool AFAST, int R1, int R2, bool CHIRP>
+__global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
+                                  (Shape<T, KIND, AFAST, R1, R2, CHIRP>::blocks))
+    fft_flex_kernel(const __grid_constant__ StageArgs A, const __grid_constant__ FlexArgs F) {
   using C = cplx<T>;
-  static constexpr bool kReal = KIND == kR2C || KIND == kC2R;
-  const StageArgs& A;
-  const FlexArgs& F;
-  C *s0, *s1;       // first / second exchange buffer
-  int b0, nb;       // first line along b, lines (real lines of R2C / C2R) in the tile
-  int nact;         // complex lines in the tile
-  int co0, co1;
+  using S = Shape<T, KIND, AFAST, R1, R2, CHIRP>;
+  constexpr bool kReal = KIND == kR2C || KIND == kC2R;
+  constexpr int B = S::B, M = S::m;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* const s = reinterpret_cast<C*>(smem_raw);
+  const int t = threadIdx.x;
+  const int per = kReal ? 2 * B : B;
+  const int b0 = static_cast<int>(blockIdx.x) * per, nb = min(per, A.Eb - b0);
+  const int nact = kReal ? (nb + 1) / 2 : nb;  // complex lines in the tile
+  const int co0 = blockIdx.y, co1 = blockIdx.z;
+  const int n = CHIRP ? F.n : M;
+  const bool inverse = KIND == kC2R || F.inverse;
+  // chirp-z of the inverse: the conjugate chirp and the filter made from it
+  auto chirp = [&](int k) {
+    C c = __ldg(reinterpret_cast<const C*>(F.chirp) + k);
+    if (inverse) c.y = -c.y;
+    return c;
+  };
+  // element e of a line
+  auto at = [&](int line, int e) -> C& { return AFAST ? s[line * S::P + e] : s[e * B + line]; };
+  constexpr int row1 = AFAST ? S::odd1 : R1, row2 = AFAST ? S::odd2 : R2;  // matrix row pitch
+  constexpr int el = AFAST ? 1 : B;                                        // pitch of neighbouring elements
 
-  // item it of cnt per line -> (line, j); false past the tile's lines
-  __device__ __forceinline__ bool split(int it, int cnt, unsigned magic, int* line, int* j) const {
-    if (AFAST) {
-      *line = static_cast<int>(__umulhi(static_cast<unsigned>(it), magic));
-      *j = it - *line * cnt;
-    } else {
-      *line = it & (F.B - 1);
-      *j = it >> F.lshift;
-    }
-    return *line < nact;
-  }
-  // items of cnt per line a tile has (a-fast: of its present lines only)
-  __device__ __forceinline__ int items(int cnt) const { return (AFAST ? nact : F.B) * cnt; }
-  // element e of a line in an exchange buffer of pitch P
-  __device__ __forceinline__ int at(int line, int e, int P) const { return AFAST ? line * P + e : e * F.B + line; }
+  // thread -> (line, j) among cnt butterflies a line
+  const int line2 = AFAST ? t / R2 : t % B, j2 = AFAST ? t % R2 : t / B;
+  const int line1 = AFAST ? t / R1 : t % B, j1 = AFAST ? t % R1 : t / B;
+  const bool act2 = (AFAST ? t < B * R2 : j2 < R2) && line2 < nact;
+  const bool act1 = (AFAST ? t < B * R1 : j1 < R1) && line1 < nact;
 
-  __device__ __forceinline__ C chirp(int k) const {
-    return __ldg(reinterpret_cast<const C*>(F.chirp) + k);
-  }
-
-  // a thread's share of a line: positions k, k + step, ... of `line`
-  __device__ __forceinline__ bool line_share(int* line, int* k, int* step) const {
-    if (AFAST) {
-      *step = F.share;
-      *line = static_cast<int>(__umulhi(threadIdx.x, F.magic_share));
-      *k = static_cast<int>(threadIdx.x) - *line * F.share;
-    } else {
-      *step = static_cast<int>(blockDim.x) >> F.lshift;
-      *line = threadIdx.x & (F.B - 1);
-      *k = static_cast<int>(threadIdx.x) >> F.lshift;
-    }
-    return *line < nact;
-  }
-
-  // value of an inverse C2C transform: real and imaginary parts swapped on the
-  // way in and out of the forward codelets
-  __device__ __forceinline__ C swapped(C c) const { return F.swap ? mk<T>(c.y, c.x) : c; }
-
-  // C2R: the full spectrum Z = X0 + i X1 of a line pair from the two half
-  // spectra (imaginary parts of DC and Nyquist dropped), parts swapped, into s1
-  __device__ __forceinline__ void assemble() const {
-    const int h = F.n / 2 + 1;
-    int line, k, step;
-    if (!line_share(&line, &k, &step)) return;
-    const C* in = reinterpret_cast<const C*>(A.in);
-    const C zero = mk<T>(T(0), T(0));
-    const bool two = 2 * line + 1 < nb;
-    const Line l0 = src_line(A, b0 + 2 * line, co0, co1);
-    const Line l1 = two ? src_line(A, b0 + 2 * line + 1, co0, co1) : l0;
-    for (; k < h; k += step) {
-      const C x0 = in[l0.at(k)];
-      const C x1 = two ? in[l1.at(k)] : zero;
-      if (k == 0 || 2 * k == F.n) {
-        s1[at(line, k, F.P1)] = mk<T>(x1.x, x0.x);
-      } else {
-        s1[at(line, k, F.P1)] = mk<T>(x0.y + x1.x, x0.x - x1.y);
-        s1[at(line, F.n - k, F.P1)] = mk<T>(x1.x - x0.y, x0.x + x1.y);
+  // ---- pass 1: codelets over positions j + r R2, row j of the matrix
+  if (act2) {
+    C v[R1];
+    if constexpr (KIND == kR2C) {
+      const T* in = reinterpret_cast<const T*>(A.in);
+#pragma unroll
+      for (int r = 0; r < R1; ++r) v[r] = mk<T>(T(0), T(0));
+      positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + 2 * line2, co0, co1), j2, n,
+                                      [&](int r, int64_t o) { v[r].x = in[o]; });
+      if (2 * line2 + 1 < nb)
+        positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + 2 * line2 + 1, co0, co1), j2, n,
+                                        [&](int r, int64_t o) { v[r].y = in[o]; });
+    } else if constexpr (KIND == kC2R) {
+      // Z = X0 + i X1 over the full line, from the two half spectra
+      // (imaginary parts of DC and Nyquist dropped)
+      const bool two = 2 * line2 + 1 < nb;
+      const C* x0 = reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2, co0, co1).base;
+      const C* x1 = two ? reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2 + 1, co0, co1).base : x0;
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        const int p = j2 + r * R2;
+        v[r] = mk<T>(T(0), T(0));
+        if (!CHIRP || p < n) {
+          const bool mirror = 2 * p > n;
+          const int q = mirror ? n - p : p;
+          C c0 = x0[q];
+          C c1 = two ? x1[q] : mk<T>(T(0), T(0));
+          if (q == 0 || 2 * q == n) {
+            v[r] = mk<T>(c0.x, c1.x);
+          } else {
+            v[r] = mirror ? mk<T>(c0.x + c1.y, c1.x - c0.y) : mk<T>(c0.x - c1.y, c0.y + c1.x);
+          }
+        }
       }
-    }
-  }
-
-  // R2C: the two half spectra of a line pair from its full spectrum in z
-  __device__ __forceinline__ void separate(const C* z, int P) const {
-    const int h = F.n / 2 + 1;
-    int line, k, step;
-    if (!line_share(&line, &k, &step)) return;
-    const T hs = T(0.5) * T(A.scale);
-    C* out = reinterpret_cast<C*>(A.out);
-    const bool two = 2 * line + 1 < nb;
-    const Line l0 = dst_line(A, b0 + 2 * line, co0, co1);
-    const Line l1 = two ? dst_line(A, b0 + 2 * line + 1, co0, co1) : l0;
-    for (; k < h; k += step) {
-      const C a = z[at(line, k, P)];
-      const C b = cconj(z[at(line, k == 0 ? 0 : F.n - k, P)]);
-      out[l0.at(k)] = cscale(cadd(a, b), hs);
-      if (two) {
-        const C d = csub(a, b);
-        out[l1.at(k)] = mk<T>(d.y * hs, -d.x * hs);
+    } else {
+      const C* in = reinterpret_cast<const C*>(A.in);
+      if (CHIRP) {
+#pragma unroll
+        for (int r = 0; r < R1; ++r) v[r] = mk<T>(T(0), T(0));
       }
+      positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + line2, co0, co1), j2, n,
+                                      [&](int r, int64_t o) { v[r] = in[o]; });
     }
-  }
-
-  // values of the R outputs v[r] at positions k0 + r * step of `line`, to the
-  // destination (C2C, C2R) or to the line's natural order in z (R2C)
-  template <int R>
-  __device__ __forceinline__ void finish(C* v, int line, int k0, int step, C* z, int P) const {
-    const int lim = F.n;
     if (CHIRP) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int k = k0 + r * step;
-        if (k < lim) v[r] = cmul(v[r], chirp(k));
-      }
+      for (int r = 0; r < R1; ++r)
+        if (j2 + r * R2 < n) v[r] = cmul(v[r], chirp(j2 + r * R2));
     }
-    if (KIND == kR2C) {
+    Dft<T, R1>::run(v);
+    C* o = &at(line2, j2 * row1);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int k = k0 + r * step;
-        if (!CHIRP || k < lim) z[at(line, k, P)] = v[r];
+    for (int r = 0; r < R1; ++r) o[r * el] = v[r];
+  }
+  __syncthreads();
+
+  const C* tw = reinterpret_cast<const C*>(F.tw);
+  const T scale = T(A.scale);
+  if constexpr (!CHIRP) {
+    // ---- pass 2: columns, outputs k = j + r R1
+    C u[R2];
+    if (act1) {
+      load_column<T, R2, R1, row1 * el>(&at(line1, j1), tw, j1, u);
+      Dft<T, R2>::run(u);
+    }
+    if constexpr (KIND == kC2C) {
+      if (act1) {
+        if (A.scale != 1.0) {
+#pragma unroll
+          for (int r = 0; r < R2; ++r) u[r] = cscale(u[r], scale);
+        }
+        C* out = reinterpret_cast<C*>(A.out);
+        outputs<R2, R1, M, AFAST>(dst_line(A, b0 + line1, co0, co1), j1, inverse,
+                                  [&](int r, int64_t o) { out[o] = u[r]; });
       }
       return;
     }
-    if (A.scale != 1.0) {
-      const T s = T(A.scale);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = cscale(v[r], s);
-    }
-    if (KIND == kC2R) {
-      T* out = reinterpret_cast<T*>(A.out);
-      const Line l0 = dst_line(A, b0 + 2 * line, co0, co1);
-      each<R, CHIRP>(l0, k0, step, lim, [&](int r, int64_t o) { out[o] = v[r].y; });
-      if (2 * line + 1 < nb) {
-        const Line l1 = dst_line(A, b0 + 2 * line + 1, co0, co1);
-        each<R, CHIRP>(l1, k0, step, lim, [&](int r, int64_t o) { out[o] = v[r].x; });
+    if constexpr (KIND == kC2R) {
+      if (act1) {
+        T* out = reinterpret_cast<T*>(A.out);
+        outputs<R2, R1, M, AFAST>(dst_line(A, b0 + 2 * line1, co0, co1), j1, true,
+                                  [&](int r, int64_t o) { out[o] = u[r].x * scale; });
+        if (2 * line1 + 1 < nb)
+          outputs<R2, R1, M, AFAST>(dst_line(A, b0 + 2 * line1 + 1, co0, co1), j1, true,
+                                    [&](int r, int64_t o) { out[o] = u[r].y * scale; });
       }
-    } else {
-      C* out = reinterpret_cast<C*>(A.out);
-      each<R, CHIRP>(dst_line(A, b0 + line, co0, co1), k0, step, lim,
-                     [&](int r, int64_t o) { out[o] = swapped(v[r]); });
+      return;
     }
-  }
-
-  // codelets over positions j + r R2 (r < R1); row j of the line's matrix
-  template <int R>
-  __device__ __forceinline__ void pass1() const {
-    const int R2 = F.R2, lim = F.n;
-    const C zero = mk<T>(T(0), T(0));
-    for (int it = threadIdx.x; it < items(R2); it += blockDim.x) {
-      int line, j;
-      if (!split(it, R2, F.magic2, &line, &j)) continue;
-      C v[R];
-      if (KIND == kC2R) {
+    __syncthreads();  // every column read: the buffer takes the line in natural order
+    if (act1) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int p = j + r * R2;
-          v[r] = (!CHIRP || p < lim) ? s1[at(line, p, F.P1)] : zero;
-        }
-      } else if (KIND == kR2C) {
-        const T* in = reinterpret_cast<const T*>(A.in);
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = zero;
-        each<R, CHIRP>(src_line(A, b0 + 2 * line, co0, co1), j, R2, lim, [&](int r, int64_t o) { v[r].x = in[o]; });
-        if (2 * line + 1 < nb)
-          each<R, CHIRP>(src_line(A, b0 + 2 * line + 1, co0, co1), j, R2, lim,
-                         [&](int r, int64_t o) { v[r].y = in[o]; });
-      } else {
-        const C* in = reinterpret_cast<const C*>(A.in);
-        if (CHIRP) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) v[r] = zero;
-        }
-        each<R, CHIRP>(src_line(A, b0 + line, co0, co1), j, R2, lim,
-                       [&](int r, int64_t o) { v[r] = swapped(in[o]); });
-      }
-      if (CHIRP) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int p = j + r * R2;
-          if (p < lim) v[r] = cmul(v[r], chirp(p));
-        }
-      }
-      Dft<T, R>::run(v);
-#pragma unroll
-      for (int r = 0; r < R; ++r) s0[at(line, j * (AFAST ? (R | 1) : R) + r, F.P0)] = v[r];
+      for (int r = 0; r < R2; ++r) at(line1, j1 + r * R1) = u[r];
     }
-  }
-
-  // columns of the R2 x R1 matrix: twiddles, codelets, outputs k = j + r R1.
-  // Chirp-z: the filter, and the first pass of the inverse transform on the
-  // same registers (its inputs are the positions j + r R1 too), row j of the
-  // R1 x R2 matrix of the way back.
-  template <int R>
-  __device__ __forceinline__ void pass2() const {
-    const int R1 = F.R1, R1p = AFAST ? (R1 | 1) : R1;
-    const C* tw = reinterpret_cast<const C*>(F.tw);
-    for (int it = threadIdx.x; it < items(R1); it += blockDim.x) {
-      int line, j;
-      if (!split(it, R1, F.magic1, &line, &j)) continue;
-      C v[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s0[at(line, r * R1p + j, F.P0)];
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(tw + r * R1 + j));
-      Dft<T, R>::run(v);
-      if (CHIRP) {
-        const C* f = reinterpret_cast<const C*>(F.filter);
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = cmul(v[r], __ldg(f + j + r * R1));
-        Dft<T, R>::run(v);  // inverse: output r is the forward output R - r
-#pragma unroll
-        for (int r = 0; r < R; ++r) s1[at(line, j * (AFAST ? (R | 1) : R) + r, F.P1)] = v[(R - r) % R];
-      } else {
-        finish<R>(v, line, j, R1, s1, F.P1);
-      }
-    }
-  }
-
-  // chirp-z: the second pass of the inverse transform, outputs k = j + r R2
-  template <int R>
-  __device__ __forceinline__ void pass3() const {
-    const int R2 = F.R2, R2p = AFAST ? (R2 | 1) : R2;
-    const C* tw = reinterpret_cast<const C*>(F.tw) + F.m;
-    for (int it = threadIdx.x; it < items(R2); it += blockDim.x) {
-      int line, j;
-      if (!split(it, R2, F.magic2, &line, &j)) continue;
-      C v[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s1[at(line, r * R2p + j, F.P1)];
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], cconj(__ldg(tw + r * R2 + j)));
-      Dft<T, R>::run(v);
-      C u[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) u[r] = v[(R - r) % R];
-      finish<R>(u, line, j, R2, s0, F.P0);
-    }
-  }
-};
-
-// codelet lengths of the register classes (class 2: the partners that the most
-// even split pairs a codelet above 16 with, 11 and 13 left out)
-#define DFFT_FLEX_R0(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10)
-#define DFFT_FLEX_R1(X) DFFT_FLEX_R0(X) X(11) X(12) X(13) X(14) X(15) X(16)
-#define DFFT_FLEX_R2(X) \
-  X(5) X(7) X(9) X(10) X(12) X(14) X(15) X(16) X(18) X(20) X(21) X(24) X(25) X(27) X(28) X(30) X(32)
-
-template <int PASS, int CLS, typename TileT>
-__device__ __forceinline__ void run_pass(const TileT& t, int R) {
-#define DFFT_CASE(R_)                       \
-  case R_:                                  \
-    if constexpr (PASS == 1)                \
-      t.template pass1<R_>();               \
-    else if constexpr (PASS == 2)           \
-      t.template pass2<R_>();               \
-    else                                    \
-      t.template pass3<R_>();               \
-    break;
-  if constexpr (CLS == 0) {
-    switch (R) { DFFT_FLEX_R0(DFFT_CASE) default: break; }
-  } else if constexpr (CLS == 1) {
-    switch (R) { DFFT_FLEX_R1(DFFT_CASE) default: break; }
   } else {
-    switch (R) { DFFT_FLEX_R2(DFFT_CASE) default: break; }
+    // ---- pass 2: columns, the filter, and the first pass of the inverse
+    // transform on the same registers (its inputs are the positions j + r R1
+    // too): row j of the R1 x R2 matrix of the way back
+    C u[R2];
+    if (act1) {
+      load_column<T, R2, R1, row1 * el>(&at(line1, j1), tw, j1, u);
+      Dft<T, R2>::run(u);
+      const C* f = reinterpret_cast<const C*>(inverse ? F.filter_inverse : F.filter);
+#pragma unroll
+      for (int r = 0; r < R2; ++r) u[r] = cmul(u[r], __ldg(f + j1 + r * R1));
+      Dft<T, R2>::run(u);  // inverse: output r is the forward output R2 - r
+    }
+    __syncthreads();
+    if (act1) {
+      C* o = &at(line1, j1 * row2);
+#pragma unroll
+      for (int r = 0; r < R2; ++r) o[r * el] = u[(R2 - r) % R2];
+    }
+    __syncthreads();
+    // ---- pass 3: outputs k = j + r R2
+    C w[R1];
+    if (act2) {
+      const C* c = &at(line2, j2);
+#pragma unroll
+      for (int r = 0; r < R1; ++r) w[r] = c[r * row2 * el];
+#pragma unroll
+      for (int r = 1; r < R1; ++r) w[r] = cmul(w[r], cconj(__ldg(tw + M + r * R2 + j2)));
+      Dft<T, R1>::run(w);
+      C x[R1];
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        x[r] = w[(R1 - r) % R1];
+        if (j2 + r * R2 < n) x[r] = cmul(x[r], chirp(j2 + r * R2));
+      }
+      if constexpr (KIND == kC2C) {
+        C* out = reinterpret_cast<C*>(A.out);
+        positions<R1, R2, AFAST, true>(dst_line(A, b0 + line2, co0, co1), j2, n,
+                                       [&](int r, int64_t o) { out[o] = cscale(x[r], scale); });
+      } else if constexpr (KIND == kC2R) {
+        T* out = reinterpret_cast<T*>(A.out);
+        positions<R1, R2, AFAST, true>(dst_line(A, b0 + 2 * line2, co0, co1), j2, n,
+                                       [&](int r, int64_t o) { out[o] = x[r].x * scale; });
+        if (2 * line2 + 1 < nb)
+          positions<R1, R2, AFAST, true>(dst_line(A, b0 + 2 * line2 + 1, co0, co1), j2, n,
+                                         [&](int r, int64_t o) { out[o] = x[r].y * scale; });
+      } else {
+#pragma unroll
+        for (int r = 0; r < R1; ++r) w[r] = x[r];
+      }
+    }
+    if constexpr (KIND != kR2C) return;
+    __syncthreads();
+    if (act2) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r)
+        if (j2 + r * R2 < n) at(line2, j2 + r * R2) = w[r];
+    }
   }
-#undef DFFT_CASE
+  // ---- R2C: the two half spectra of a line pair from its full spectrum
+  if constexpr (KIND == kR2C) {
+    __syncthreads();
+    constexpr int TPL = S::NT / B;  // threads a line
+    const int line = t / TPL;
+    if (line < nact) {
+      C* out = reinterpret_cast<C*>(A.out);
+      const T hs = T(0.5) * scale;
+      const bool two = 2 * line + 1 < nb;
+      C* y0 = out + dst_line(A, b0 + 2 * line, co0, co1).base;
+      C* y1 = two ? out + dst_line(A, b0 + 2 * line + 1, co0, co1).base : y0;
+      for (int k = t % TPL; k <= n / 2; k += TPL) {
+        const C a = at(line, k);
+        const C b = cconj(at(line, k == 0 ? 0 : n - k));
+        y0[k] = cscale(cadd(a, b), hs);
+        if (two) {
+          const C d = csub(a, b);
+          y1[k] = mk<T>(d.y * hs, -d.x * hs);
+        }
+      }
+    }
+  }
 }
 
-template <typename T, int KIND, bool AFAST, int CLS, bool CHIRP>
-__global__ void __launch_bounds__(Bounds<T, CLS>::threads, (Bounds<T, CLS>::blocks))
-    fft_flex_kernel(const __grid_constant__ StageArgs A, const __grid_constant__ FlexArgs F) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  using TileT = Tile<T, KIND, AFAST, CHIRP>;
-  using C = cplx<T>;
-  const int per = TileT::kReal ? 2 * F.B : F.B;
-  const int b0 = static_cast<int>(blockIdx.x) * per, nb = min(per, A.Eb - b0);
-  C* s0 = reinterpret_cast<C*>(smem_raw);
-  const TileT t{A, F, s0, s0 + F.B * F.P0, b0, nb, TileT::kReal ? (nb + 1) / 2 : nb,
-                static_cast<int>(blockIdx.y), static_cast<int>(blockIdx.z)};
-  if (KIND == kC2R) {
-    t.assemble();
-    __syncthreads();
-  }
-  run_pass<1, CLS>(t, F.R1);
-  __syncthreads();
-  run_pass<2, CLS>(t, F.R2);
-  if (CHIRP) {
-    __syncthreads();
-    run_pass<3, CLS>(t, F.R1);
-  }
-  if (KIND == kR2C) {
-    __syncthreads();
-    t.separate(CHIRP ? t.s0 : t.s1, CHIRP ? F.P0 : F.P1);
-  }
-}
+using LaunchFn = cudaError_t (*)(const StageArgs& A, const FlexArgs& F, cudaStream_t st);
 
-template <typename T, int KIND, bool AFAST, int CLS, bool CHIRP>
+template <typename T, int KIND, bool AFAST, int R1, int R2, bool CHIRP>
 cudaError_t launch_kernel(const StageArgs& A, const FlexArgs& F, cudaStream_t st) {
-  auto k = fft_flex_kernel<T, KIND, AFAST, CLS, CHIRP>;
-  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), F.smem);
+  using S = Shape<T, KIND, AFAST, R1, R2, CHIRP>;
+  auto k = fft_flex_kernel<T, KIND, AFAST, R1, R2, CHIRP>;
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), S::smem);
   if (e != cudaSuccess) return e;
-  k<<<fast_grid(A), F.nthreads, F.smem, st>>>(with_table_offsets(A), F);
+  k<<<fast_grid(A), S::NT, S::smem, st>>>(with_table_offsets(A), F);
   return cudaGetLastError();
 }
 
-// The kernels of one precision, register class and form: instantiated by
-// fft_flex_inst.cu, one translation unit each.  Real lines are a-fast only.
-template <typename T, int CLS, bool CHIRP>
-cudaError_t launch_class(const StageArgs& A, const FlexArgs& F, int kind, cudaStream_t st);
+// The kernels of one length: C2C a-fast and b-fast, R2C and C2R (a-fast).
+struct Entry {
+  int m;
+  LaunchFn c2c_a, c2c_b, r2c, c2r;
+};
+// The entries of one group of lengths (fft_flex_lengths.h), defined by
+// fft_flex_inst.cu in a translation unit each.
+template <typename T, bool CHIRP, int GROUP>
+struct Group {
+  static const Entry* entries(int* count);
+};
 
 }  // namespace flex
 }  // namespace dev

@@ -412,27 +412,26 @@ const void* Plan::flex_twiddle(int r1, int r2) {
   return p;
 }
 
-void Plan::select_flex(Op& op, int opt) const {
-  const dev::FlexArgs& F = op.flex.at(opt);
-  op.flex_opt = opt;
+void Plan::select_flex(Op& op) const {
   dev::StageArgs& A = op.sa;
   A.pairs = 4;
-  A.B = F.B;
-  const int per = op.kind == dev::kC2C ? F.B : 2 * F.B;
+  A.B = op.flex_B;
+  const int per = op.kind == dev::kC2C ? A.B : 2 * A.B;
   A.tiles_b = (A.Eb + per - 1) / per;
   op.tiles = static_cast<unsigned>(static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1);
 }
 
-// The two-pass kernel's options of a stage whose geometry (axes, extents, row
-// orientation) is set: lengths that split into two codelets, or whose chirp-z
-// convolution does; rows of one orientation on both sides (R2C / C2R: along
-// a); every side addressable by line (separable tables, or general ones whose
-// rank blocks do not split a).  Fills op.flex and the line addressing; false
-// (op untouched) if the kernel does not take the stage.
+// The two-pass kernel for a stage whose geometry (axes, extents, row
+// orientation) is set: lengths that have a kernel (fft_flex_lengths.h), or
+// whose chirp-z convolution does; rows of one orientation on both sides; every
+// side addressable by line: separable tables (R2C / C2R: lines in one piece),
+// or general ones whose rank blocks do not split a.  Fills op.fx and the line
+// addressing; false (op untouched) if the kernel does not take the stage.
 bool Plan::add_flex(Op& op) {
   dev::StageArgs& A = op.sa;
   const std::size_t a = static_cast<std::size_t>(A.a);
-  if (A.load_afast != A.store_afast || A.Eo0 > dev::fast_stage_max_grid_yz() ||
+  const bool real = op.kind != dev::kC2C, afast = A.load_afast != 0;
+  if (A.load_afast != A.store_afast || (real && !afast) || A.Eo0 > dev::fast_stage_max_grid_yz() ||
       A.Eo1 > dev::fast_stage_max_grid_yz())
     return false;
   const int nh = A.n / 2 + 1;
@@ -444,19 +443,27 @@ bool Plan::add_flex(Op& op) {
   for (int k = 0; k < 2; ++k) {
     const int l = k == 0 ? op.src_layout : op.dst_layout;
     const LayoutTables& T = tables_[l];
+    const std::size_t len = layouts_[l].gext[a];
     Side& s = side[k];
+    // the kernels take the offsets along a line (32 bits), unit stride when a-fast
+    if (afast && layout_fast_axis(layouts_[l]) != a) return false;
     if (T.mode != 0) {
       if (layouts_[l].topo[a] != 1) return false;
       s.affine = 1;
+      for (const RankBlock& rb : layout_blocks(layouts_[l]))
+        if (static_cast<std::int64_t>(len) * static_cast<std::int64_t>(rb.stride[a]) >= (std::int64_t(1) << 31))
+          return false;
       continue;
     }
-    const std::size_t len = layouts_[l].gext[a];
     const std::int64_t* off = T.data.data() + T.off[a];
     s.stride = len > 1 ? off[1] - off[0] : 1;
     s.base = off[0];
     for (std::size_t c = 1; c < len; ++c)
       if (off[c] != off[0] + static_cast<std::int64_t>(c) * s.stride) s.atab = 1;
+    if (afast && s.stride != 1) s.atab = 1;
+    if (s.stride < 0 || static_cast<std::int64_t>(len) * s.stride >= (std::int64_t(1) << 31)) s.atab = 1;
     if (s.atab) {
+      if (real) return false;
       s.base = 0;  // the table carries the whole offset along a
       s.stride = 1;
     }
@@ -464,24 +471,18 @@ bool Plan::add_flex(Op& op) {
   int r1 = 0, r2 = 0;
   const bool chirp = !radix_supported(static_cast<std::size_t>(A.n));
   const int m = chirp ? dev::flex_chirp_length(A.n) : A.n;
-  if (m == 0 || !dev::flex_split(m, &r1, &r2)) return false;
-  std::vector<dev::FlexArgs> opts;
-  for (int o = 0; o < dev::kFlexOptions; ++o) {
-    dev::FlexArgs F;
-    if (!dev::flex_config(d_.dbl, op.kind, A.load_afast != 0, A.n, m, o, &F)) continue;
-    const int per = op.kind == dev::kC2C ? F.B : 2 * F.B;
-    if (static_cast<unsigned long long>((A.Eb + per - 1) / per) * A.Eo0 * A.Eo1 >= (1ull << 31)) continue;
-    opts.push_back(F);
-  }
-  if (opts.empty()) return false;
-  const void *ch = nullptr, *filt = nullptr, *finv = nullptr;
-  if (chirp) bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &ch, &filt, &finv);
-  for (auto& F : opts) {
-    F.tw = flex_twiddle(F.R1, F.R2);
-    F.chirp = ch;
-    F.filter = filt;
-  }
-  op.flex = opts;
+  if (m == 0 || !dev::flex_split(m, chirp, &r1, &r2)) return false;
+  const int B = dev::flex_lines(d_.dbl, afast, r1), per = real ? 2 * B : B;
+  if (static_cast<unsigned long long>((A.Eb + per - 1) / per) * A.Eo0 * A.Eo1 >= (1ull << 31)) return false;
+  op.flex = true;
+  op.flex_B = B;
+  op.fx = dev::FlexArgs{};
+  op.fx.n = A.n;
+  op.fx.m = m;
+  op.fx.tw = flex_twiddle(r1, r2);
+  if (chirp)
+    bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &op.fx.chirp, &op.fx.filter,
+                     &op.fx.filter_inverse);
   A.src_line_affine = side[0].affine;
   A.src_atab = side[0].atab;
   A.src_abase = side[0].base;
@@ -693,7 +694,7 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
   if (!is_copy && !radix_supported(n)) {
     op.chirp = true;
     if (add_flex(op)) {
-      select_flex(op, 0);
+      select_flex(op);
       return op;
     }
     // chirp-z stage: a circular convolution of length m >= 2n - 1
@@ -887,7 +888,7 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
     // same line addressing)
     if (!A.comp) add_flex(op);
   } else if (!is_copy && add_flex(op)) {
-    select_flex(op, 0);
+    select_flex(op);
   }
   return op;
 }
@@ -982,7 +983,7 @@ static cudaError_t launch_fast_op(const dev::StageArgs& A, bool dbl, int kind, b
 // TMA kernel needs a source the tensor map can address (16-byte aligned
 // pointer); the two-line b-fast kernels need 16-byte aligned buffers.
 cudaError_t Plan::launch_stage(const Op& op, dev::StageArgs A, cudaStream_t stream) const {
-  if (A.pairs == 4) return dev::launch_fft_flex(A, op.flex[op.flex_opt], d_.dbl, op.kind, op.inverse, stream);
+  if (A.pairs == 4) return dev::launch_fft_flex(A, op.fx, d_.dbl, op.kind, op.inverse, stream);
   if (!op.fast) return dev::launch_fft_stage(A, d_.dbl, op.kind, op.inverse, op.nthreads, op.smem, op.tiles, stream);
   const bool misaligned = ((reinterpret_cast<std::uintptr_t>(A.in) | reinterpret_cast<std::uintptr_t>(A.out)) & 15) != 0;
   if (A.pairs == 3) {
@@ -1469,7 +1470,7 @@ void Plan::autotune() {
   load_tune_cache_locked();
   for (auto* progs : {&prog_[0], &prog_[1], &adj_[0], &adj_[1]}) {
     for (auto& op : *progs) {
-      if (op.type != Op::Stage || (!op.fast && op.flex.empty())) continue;
+      if (op.type != Op::Stage || !op.fast) continue;
       dev::StageArgs& A = op.sa;
 
       // Trial buffers: the op's own plan-owned buffers, else the scratch
@@ -1489,7 +1490,7 @@ void Plan::autotune() {
       const bool real = op.kind == dev::kR2C || op.kind == dev::kC2R;  // two real lines per register line
       const bool pair_ok = op.single_B != 0;                            // eligible for two lines per thread
       const bool tma_ok = op.tma.ok;                                    // eligible for the TMA-fed kernel
-      k << (op.flex.empty() ? "fast:n" : op.fast ? "fast+flex:n" : "flex:n") << A.n << (d_.dbl ? "f64" : "f32") << (op.inverse ? "i" : "f") << (A.load_afast ? "a" : "b")
+      k << (op.flex ? "fast+flex:n" : "fast:n") << A.n << (d_.dbl ? "f64" : "f32") << (op.inverse ? "i" : "f") << (A.load_afast ? "a" : "b")
         << (op.kind == dev::kR2C ? "r2c" : op.kind == dev::kC2R ? "c2r" : "") << (pair_ok ? "P" : "")
         << (tma_ok ? "T" : "") << (A.comp ? "C" : "")
         << (A.src_line_affine || A.dst_line_affine || A.src_atab || A.dst_atab ? "G" : "") << ":" << A.Eb << "x"
@@ -1506,12 +1507,11 @@ void Plan::autotune() {
       // a configuration: lines per tile of the one-line kernel; kPairCode +
       // lines per tile of the two-line kernel; kStreamCode + tiles per CTA of
       // its streaming variant; kTmaCode + lines per tile of the TMA-fed
-      // kernel; kFlexCode + option of the two-pass kernel
+      // kernel; kFlexCode the two-pass kernel
       constexpr int kPairCode = 100000, kStreamCode = 200000, kTmaCode = 300000, kFlexCode = 400000;
-      const int nflex = static_cast<int>(op.flex.size());
       auto apply = [&](int code) {
         if (code >= kFlexCode) {
-          select_flex(op, code - kFlexCode);
+          select_flex(op);
           return;
         }
         if (code >= kTmaCode) {
@@ -1530,9 +1530,9 @@ void Plan::autotune() {
       };
       auto it = g_tune_cache.find(key);
       if (it != g_tune_cache.end() &&
-          (it->second >= kFlexCode ? it->second - kFlexCode < nflex
-                                   : op.fast && (it->second < kPairCode || pair_ok) &&
-                                         (it->second < kTmaCode || tma_ok))) {
+          (it->second >= kFlexCode
+               ? op.flex
+               : (it->second < kPairCode || pair_ok) && (it->second < kTmaCode || tma_ok))) {
         apply(it->second);
         continue;
       }
@@ -1567,10 +1567,10 @@ void Plan::autotune() {
         for (int tpc : {4, 8, 16})
           if (tiles >= 2 * tpc) cand.push_back(kStreamCode + tpc);
       }
-      const int nopt = A.comp || !op.fast ? 0 : dev::fast_stage_line_options(d_.dbl, A.n, opts);
+      const int nopt = A.comp ? 0 : dev::fast_stage_line_options(d_.dbl, A.n, opts);
       for (int i = 0; i < nopt; ++i) cand.push_back(opts[i]);
-      for (int i = 0; i < nflex; ++i) cand.push_back(kFlexCode + i);
-      int best = A.pairs == 4 ? kFlexCode + op.flex_opt : A.pairs == 3 ? kTmaCode + A.B : A.pairs == 2 ? kStreamCode + A.tpc : (A.pairs ? kPairCode : 0) + A.B;
+      if (op.flex) cand.push_back(kFlexCode);
+      int best = A.pairs == 4 ? kFlexCode : A.pairs == 3 ? kTmaCode + A.B : A.pairs == 2 ? kStreamCode + A.tpc : (A.pairs ? kPairCode : 0) + A.B;
       float best_ms = std::numeric_limits<float>::max();
       cudaEvent_t e0, e1;
       cuda_check(cudaEventCreate(&e0), "tuner event");
@@ -1584,12 +1584,18 @@ void Plan::autotune() {
           cudaGetLastError();
           continue;
         }
-        cudaEventRecord(e0, st);
-        for (int r = 0; r < 3; ++r) launch_stage(op, T, st);
-        cudaEventRecord(e1, st);
-        cuda_check(cudaEventSynchronize(e1), "tuner sync");
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
+        auto timed = [&](int reps) {
+          cudaEventRecord(e0, st);
+          for (int r = 0; r < reps; ++r) launch_stage(op, T, st);
+          cudaEventRecord(e1, st);
+          cuda_check(cudaEventSynchronize(e1), "tuner sync");
+          float ms = 0.f;
+          cudaEventElapsedTime(&ms, e0, e1);
+          return ms / static_cast<float>(reps);
+        };
+        // short launches again: three of them measure the launch gaps too
+        float ms = timed(3);
+        if (ms < 0.05f) ms = std::min(timed(10), timed(10));
         if (ms < best_ms) {
           best_ms = ms;
           best = code;

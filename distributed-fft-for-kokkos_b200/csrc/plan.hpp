@@ -83,10 +83,11 @@ struct Op {
                       // caller buffers turn out not to be 16-byte aligned
   int pair_B = 0;     // lines per tile of the two-line kernel, for TMA stages whose source
                       // cannot be described by a tensor map at run time
-  // two-pass kernel (fft_flex.cuh): its options (tile and radix order), the one
-  // in use; a register stage (fast) may run it too when the tuner picks it
-  std::vector<dev::FlexArgs> flex;
-  int flex_opt = 0;
+  // two-pass kernel (fft_flex.cuh): the only kernel of the stage, or (fast) one
+  // the tuner may pick; flex_B complex lines per tile
+  bool flex = false;
+  dev::FlexArgs fx{};
+  int flex_B = 0;
   TmaSource tma;      // source description of a TMA-eligible b-fast pair stage
   // chirp-z stage (line length with a prime factor above 13): make_stage marks
   // it, push_stage expands it into pre / FFT / mul / inverse FFT / post ops
@@ -221,7 +222,7 @@ class Plan {
   // Twiddles of an m = R1 R2 point two-pass stage (dev::FlexArgs::tw).
   std::map<std::pair<int, int>, void*> flex_tables_;
   const void* flex_twiddle(int r1, int r2);
-  void select_flex(Op& op, int opt) const;
+  void select_flex(Op& op) const;
   bool add_flex(Op& op);
   std::int64_t add_geo(const Layout& L, const BlockInfo& b, std::size_t pc);
   void build_fused(bool forward);
