@@ -53,7 +53,10 @@ __global__ void blue_pre_kernel(const BlueArgs B) {
         c[S.a] = mirror ? n - j : j;
         v = reinterpret_cast<const C*>(S.in)[layout_offset(S.src, c, S.nd)];
         if (mirror) v.y = -v.y;
-        if (j == 0 || 2 * j == n) v.y = T(0);
+        if (j == 0 || 2 * j == n)
+          v.y = T(0);
+        else
+          v = cscale(v, T(S.weight));
       } else {
         c[S.a] = j;
         v = reinterpret_cast<const C*>(S.in)[layout_offset(S.src, c, S.nd)];
@@ -107,7 +110,8 @@ __global__ void blue_post_kernel(const BlueArgs B) {
     const long long line = i / nout;
     const int k = static_cast<int>(i % nout);
     const long long src = B.four_n1 > 0 ? (k % B.four_n2) * static_cast<long long>(B.four_n1) + k / B.four_n2 : k;
-    const C v = cscale(cmul(z[line * m + src], chirp_at<T>(B, k)), sc);
+    C v = cscale(cmul(z[line * m + src], chirp_at<T>(B, k)), sc);
+    if (B.kind == kR2C && k != 0 && 2 * k != n) v = cscale(v, T(S.weight));
     int c[4];
     line_coords(S, line, c);
     c[S.a] = k;

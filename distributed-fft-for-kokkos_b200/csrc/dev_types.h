@@ -35,6 +35,7 @@ struct StageArgs {
   int tiles_b;        // ceil(Eb / B)
   int load_afast, store_afast;  // thread order of the gather / scatter
   double scale;                 // applied on store
+  double weight;                // R2C / C2R: factor of the interior modes (k != 0, 2 k != n)
   int npass;
   unsigned long long radix_code;  // radix of pass p in bits [4p, 4p+4)
   // register kernels: 1 = address each line as base + p * stride, both taken
@@ -226,10 +227,6 @@ cudaError_t launch_bluestein(int op, const BlueArgs& B, bool dbl, cudaStream_t s
 // op: 0 pack, 1 all-to-all, 2 unpack
 cudaError_t launch_xpose(int op, const XposeArgs& X, int elem_bytes, cudaStream_t st);
 cudaError_t launch_scale(void* p, int64_t n_real, bool dbl, double s, cudaStream_t st);
-// Multiply the interior modes (k != 0, 2k != n_real along `axis`) of a complex
-// array stored in layout L by `factor`.
-cudaError_t launch_weight(const DevLayout& L, void* data, bool dbl, int nd, const int64_t* ext, int axis, int n_real,
-                          double factor, cudaStream_t st);
 
 }  // namespace dev
 }  // namespace dfft

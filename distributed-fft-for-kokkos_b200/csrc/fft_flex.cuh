@@ -243,6 +243,8 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
           if (q == 0 || 2 * q == n) {
             v[r] = mk<T>(c0.x, c1.x);
           } else {
+            c0 = cscale(c0, T(A.weight));
+            c1 = cscale(c1, T(A.weight));
             v[r] = mirror ? mk<T>(c0.x + c1.y, c1.x - c0.y) : mk<T>(c0.x - c1.y, c0.y + c1.x);
           }
         }
@@ -371,13 +373,14 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
     const int line = t / TPL;
     if (line < nact) {
       C* out = reinterpret_cast<C*>(A.out);
-      const T hs = T(0.5) * scale;
+      const T h0 = T(0.5) * scale, h1 = h0 * T(A.weight);
       const bool two = 2 * line + 1 < nb;
       C* y0 = out + dst_line(A, b0 + 2 * line, co0, co1).base;
       C* y1 = two ? out + dst_line(A, b0 + 2 * line + 1, co0, co1).base : y0;
       for (int k = t % TPL; k <= n / 2; k += TPL) {
         const C a = at(line, k);
         const C b = cconj(at(line, k == 0 ? 0 : n - k));
+        const T hs = (k == 0 || 2 * k == n) ? h0 : h1;
         y0[k] = cscale(cadd(a, b), hs);
         if (two) {
           const C d = csub(a, b);

@@ -282,12 +282,14 @@ __global__ void __launch_bounds__(256) fft_stage_kernel(const StageArgs A) {
     const int total = A.nl * h;
     for (int it = threadIdx.x; it < total; it += nt) {
       const int m = it / h, k = it - m * h;
-      const C x0 = buf0[m * A.pitch + k];
-      const C x1 = buf0[m * A.pitch + h + k];
+      C x0 = buf0[m * A.pitch + k];
+      C x1 = buf0[m * A.pitch + h + k];
       C* line = buf1 + m * A.pitch;
       if (k == 0 || 2 * k == A.n) {
         line[k] = mk<T>(x0.x, x1.x);
       } else {
+        x0 = cscale(x0, T(A.weight));
+        x1 = cscale(x1, T(A.weight));
         line[k] = mk<T>(x0.x - x1.y, x0.y + x1.x);
         line[A.n - k] = mk<T>(x0.x + x1.y, x1.x - x0.y);
       }
@@ -334,12 +336,13 @@ __global__ void __launch_bounds__(256) fft_stage_kernel(const StageArgs A) {
         const C* zl = cur + (line >> 1) * A.pitch;
         const C z = zl[pos];
         const C zc = cconj(zl[pos == 0 ? 0 : A.n - pos]);
+        const T hs = T(0.5) * s * ((pos == 0 || 2 * pos == A.n) ? T(1) : T(A.weight));
         C x;
         if ((line & 1) == 0) {
-          x = cscale(cadd(z, zc), T(0.5) * s);
+          x = cscale(cadd(z, zc), hs);
         } else {
           const C d = csub(z, zc);
-          x = mk<T>(d.y * (T(0.5) * s), -d.x * (T(0.5) * s));
+          x = mk<T>(d.y * hs, -d.x * hs);
         }
         reinterpret_cast<C*>(A.out)[o] = x;
       } else if (KIND == kC2R) {

@@ -220,6 +220,7 @@ __device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, i
 //   C2R: Z[k] = X0[k] + i X1[k] and Z[N-k] = conj X0[k] + i conj X1[k] are
 //        assembled in shared memory (imaginary parts of DC and Nyquist
 //        dropped), inverse FFT, x0 = Re z and x1 = Im z are written.
+// The interior modes (all but DC and Nyquist) carry the factor A.weight.
 template <typename T, bool C2R, int N, int B, bool AFF>
 __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw,
                                           bool stage_tw = true) {
@@ -271,7 +272,7 @@ __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, i
     drow0 = dof + (act0 ? __ldg(ld.t + A.d_tb + b0 + r0) : 0);
     drow1 = dof + (act1 ? __ldg(ld.t + A.d_tb + b0 + r1) : 0);
   }
-  const T s = T(A.scale);
+  const T s = T(A.scale), wt = T(A.weight);
   // position p of a line -> offset from its row base: p, or (general-layout
   // variant, a side split into bins along a) the axis table
   const bool satab = AFF && A.src_atab, datab = AFF && A.dst_atab;
@@ -298,11 +299,13 @@ __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, i
     const C* row1 = in + srow1;
     for (int k = t; k <= H; k += TT) {
       const int64_t pk = spos(k);
-      const C x0 = act0 ? row0[pk] : mk<T>(T(0), T(0));
-      const C x1 = act1 ? row1[pk] : mk<T>(T(0), T(0));
+      C x0 = act0 ? row0[pk] : mk<T>(T(0), T(0));
+      C x1 = act1 ? row1[pk] : mk<T>(T(0), T(0));
       if (k == 0 || k == H) {
         ln[padpos<S>(k)] = mk<T>(x0.x, x1.x);
       } else {
+        x0 = cscale(x0, wt);
+        x1 = cscale(x1, wt);
         ln[padpos<S>(k)] = mk<T>(x0.x - x1.y, x0.y + x1.x);
         ln[padpos<S>(N - k)] = mk<T>(x0.x + x1.y, x1.x - x0.y);
       }
@@ -328,8 +331,9 @@ __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, i
     C* out = reinterpret_cast<C*>(A.out);
     C* row0 = out + drow0;
     C* row1 = out + drow1;
-    const T hs = T(0.5) * s;
+    const T h0 = T(0.5) * s, h1 = h0 * wt;
     for (int k = t; k <= H; k += TT) {
+      const T hs = (k == 0 || k == H) ? h0 : h1;
       const C z = ln[padpos<S>(k)];
       const C zc = cconj(ln[padpos<S>(k == 0 ? 0 : N - k)]);
       const int64_t pk = dpos(k);

@@ -690,6 +690,7 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
   A.load_afast = fs == a ? 1 : 0;
   A.store_afast = fd == a ? 1 : 0;
   A.scale = scale;
+  A.weight = 1.0;
 
   if (!is_copy && !radix_supported(n)) {
     op.chirp = true;
@@ -1057,8 +1058,9 @@ void Plan::build_fused(bool forward) {
 // R2C (real x, half spectrum along the R2C axis): adjoint(R2C) = C2R * diag(1/w)
 // and adjoint(C2R) = diag(w) * R2C with w = 2 on the interior modes (doubled by
 // the Hermitian extension) and 1 on DC / Nyquist; the weights commute with the
-// C2C transforms along the other axes and are applied to a complex
-// intermediate through the layout tables.
+// C2C transforms along the other axes and are factors in the load of the C2R
+// stage and the store of the R2C stage (StageArgs::weight; powers of two, so
+// exact wherever they are applied).
 // ---------------------------------------------------------------------------
 void Plan::build_adjoint(bool of_forward) {
   auto& prog = adj_[of_forward ? 0 : 1];
@@ -1074,40 +1076,21 @@ void Plan::build_adjoint(bool of_forward) {
   I.complex = true;
   const int li = add_layout(I), lin = add_layout(lin_), lout = add_layout(lout_);
   const double scale = of_forward ? scale_fwd_ : scale_bwd_;
-  auto weight_op = [&](int layout, int buf, double factor) {
-    Op w;
-    w.type = Op::Weight;
-    w.src = w.dst = buf;
-    w.src_layout = layout;
-    w.w_axis = static_cast<int>(ar);
-    w.w_n = static_cast<int>(d_.gin[ar]);
-    w.scale = factor;
-    return w;
-  };
   if (of_forward) {
     // output layout -> input layout: inverse transforms, C2R last
     std::reverse(order.begin(), order.end());
     int cur_l = lout, cur_b = kBufIn;
-    if (d_.r2c && S == 1) {
-      Op c = make_stage(lout, li, layout_fast_axis(lout_), dev::kCopy, false, 1.0);
-      c.src = kBufIn;
-      c.dst = kBufScratch0;
-      prog.push_back(c);
-      prog.push_back(weight_op(li, kBufScratch0, 0.5));
-      cur_l = li;
-      cur_b = kBufScratch0;
-    }
     for (std::size_t s = 0; s < S; ++s) {
       const bool last = s == S - 1;
       const int kind = (last && d_.r2c) ? dev::kC2R : dev::kC2C;
       const int dst_l = last ? lin : li;
       Op op = make_stage(cur_l, dst_l, order[s], kind, true, last ? scale : 1.0);
+      if (kind == dev::kC2R) op.sa.weight = 0.5;
       op.src = cur_b;
       op.dst = last ? kBufOut : (cur_b == kBufScratch0 ? kBufScratch1 : kBufScratch0);
       push_stage(prog, op);
       cur_l = dst_l;
       cur_b = op.dst;
-      if (s == 0 && d_.r2c && S >= 2) prog.push_back(weight_op(li, cur_b, 0.5));
     }
   } else {
     // input layout -> output layout: forward transforms, R2C first
@@ -1117,12 +1100,12 @@ void Plan::build_adjoint(bool of_forward) {
       const int kind = (first && d_.r2c) ? dev::kR2C : dev::kC2C;
       const int dst_l = last ? lout : li;
       Op op = make_stage(cur_l, dst_l, order[s], kind, false, last ? scale : 1.0);
+      if (kind == dev::kR2C) op.sa.weight = 2.0;
       op.src = cur_b;
       op.dst = last ? kBufOut : (cur_b == kBufScratch0 ? kBufScratch1 : kBufScratch0);
       push_stage(prog, op);
       cur_l = dst_l;
       cur_b = op.dst;
-      if (first && d_.r2c) prog.push_back(weight_op(cur_l, cur_b, 2.0));
     }
   }
 }
@@ -1412,7 +1395,6 @@ void Plan::allocate_device() {
   };
   for (auto* progs : {&prog_[0], &prog_[1], &adj_[0], &adj_[1]}) {
     for (auto& op : *progs) {
-      if (op.type == Op::Weight) op.sa.dst = dev_layout(op.src_layout);
       if (op.type == Op::Stage || op.type == Op::BluePre || op.type == Op::BluePost) {
         op.sa.src = dev_layout(op.src_layout);
         op.sa.dst = dev_layout(op.dst_layout);
@@ -1678,14 +1660,6 @@ void Plan::run_program(const std::vector<Op>& prog, const void* in, void* out, c
       }
       case Op::Scale: e = dev::launch_scale(buf(op0.dst), op0.n_real, d_.dbl, op0.scale, stream); break;
       case Op::Copy: e = cudaMemcpyAsync(buf(op0.dst), buf(op0.src), op0.bytes, cudaMemcpyDeviceToDevice, stream); break;
-      case Op::Weight: {
-        const Layout& L = layouts_[op0.src_layout];
-        std::int64_t ext[4] = {1, 1, 1, 1};
-        for (std::size_t k = 0; k < L.gext.size(); ++k) ext[k] = static_cast<std::int64_t>(L.gext[k]);
-        e = dev::launch_weight(op0.sa.dst, buf(op0.dst), d_.dbl, static_cast<int>(L.gext.size()), ext, op0.w_axis,
-                               op0.w_n, op0.scale, stream);
-        break;
-      }
     }
     if (e != cudaSuccess) fail(kErrCuda, std::string("kernel launch failed: ") + cudaGetErrorString(e));
   }

@@ -72,7 +72,7 @@ bool tma_encode(void* map, const void* base, const TmaSource& t);
 std::vector<double> two_pass_twiddles(int r1, int r2);
 
 struct Op {
-  enum Type { Stage, Pack, All2All, Unpack, Scale, Copy, Weight, BluePre, BlueMul, BluePost, FourTwiddle } type;
+  enum Type { Stage, Pack, All2All, Unpack, Scale, Copy, BluePre, BlueMul, BluePost, FourTwiddle } type;
   int src = -1, dst = -1;  // buffer ids
   // Stage
   dev::StageArgs sa{};
@@ -110,8 +110,6 @@ struct Op {
   dev::XposeArgs xa{};
   int elem_bytes = 0;
   int block = -1;  // transpose block index in the block list
-  // Weight (Hermitian weights of an R2C spectrum)
-  int w_axis = 0, w_n = 0;
   // Scale / Copy
   std::int64_t n_real = 0;
   std::size_t bytes = 0;
