@@ -8,15 +8,18 @@
 //   -adv - nu k^2 u_hat (:655-669); projection u - k (k . u) / k^2 (:241-260);
 //   RK4 low-storage stages (examples/utils/math_utils.hpp:90-141).
 //
-// Every kernel walks global coordinates and addresses the rank-blocked
-// buffers through the plan's layout tables, so the spectral operators see the
-// global wavenumber of each element whatever the topology.  The RK4 stage
-// update is fused into the combine / projection kernel.
+// The right-hand side runs on spectra of the modes the 2/3 rule keeps, in
+// arrays of its own (ns_lines.cuh); the caller's rank-blocked spectra are read
+// and written once per call, through the plan's layout tables.  Grids those
+// kernels do not take run the transforms of the plan around pointwise kernels
+// that walk global coordinates, with the RK4 stage update fused into the
+// combine / projection kernel.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <vector>
+#include <memory>
 #include <new>
 #include <string>
 
@@ -25,6 +28,7 @@
 #include "batch.hpp"
 #include "layout.hpp"
 #include "ns.hpp"
+#include "ns_lines.hpp"
 
 #include <algorithm>
 #include "plan.hpp"
@@ -464,6 +468,71 @@ __global__ void ns_adj_combine_kernel(const DevLayout L, const cplx<T>* mu, cons
   }
 }
 
+// ---- spectra of kept modes, (3, kx, ky, kz): index i of an axis with n
+// points and cutoff c is mode i (i <= c) or i - (2 c + 1) ----
+
+struct NsKept {
+  int kx, ky, kz;  // kept modes per axis
+};
+
+// kept modes of a caller's spectrum
+template <typename T>
+__global__ void ns_gather_kernel(const DevLayout L, const cplx<T>* uk, cplx<T>* a, NsGeom g, NsKept k) {
+  const int64_t total = static_cast<int64_t>(k.kx) * k.ky * k.kz;
+  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int ix, iy, iz;
+    decode_point(t, k.kz, k.ky, &ix, &iy, &iz);
+    int64_t o[3];
+    off3(L, ix <= g.cx ? ix : ix - k.kx + g.nx, iy <= g.cy ? iy : iy - k.ky + g.ny, iz, o);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[d * total + t] = uk[o[d]];
+  }
+}
+
+// the caller's spectrum from kept modes, zero elsewhere
+template <typename T>
+__global__ void ns_scatter_kernel(const DevLayout L, const cplx<T>* a, cplx<T>* uk, NsGeom g, NsKept k) {
+  const int64_t total = static_cast<int64_t>(g.nx) * g.ny * g.nzh, nk = static_cast<int64_t>(k.kx) * k.ky * k.kz;
+  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int ix, iy, iz;
+    decode_point(t, g.nzh, g.ny, &ix, &iy, &iz);
+    const int jx = ix <= g.cx ? ix : (ix >= g.nx - g.cx ? ix - g.nx + k.kx : -1);
+    const int jy = iy <= g.cy ? iy : (iy >= g.ny - g.cy ? iy - g.ny + k.ky : -1);
+    const bool keep = jx >= 0 && jy >= 0 && iz <= g.cz;
+    const int64_t e = (static_cast<int64_t>(jx) * k.ky + jy) * k.kz + iz;
+    int64_t o[3];
+    off3(L, ix, iy, iz, o);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) uk[o[d]] = keep ? a[d * nk + e] : mk<T>(T(0), T(0));
+  }
+}
+
+// mu = P c on kept modes
+template <typename T>
+__global__ void ns_kept_project_kernel(const cplx<T>* c, cplx<T>* mu, NsGeom g, NsKept k) {
+  const int64_t total = static_cast<int64_t>(k.kx) * k.ky * k.kz;
+  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int ix, iy, iz;
+    decode_point(t, k.kz, k.ky, &ix, &iy, &iz);
+    const double kx = (ix <= g.cx ? ix : ix - k.kx) * g.kscale, ky = (iy <= g.cy ? iy : iy - k.ky) * g.kscale,
+                 kz = iz * g.kscale;
+    const double inv_ksq = t == 0 ? 0.0 : 1.0 / (kx * kx + ky * ky + kz * kz);
+    const T ikk = T(inv_ksq);
+    const T kk[3] = {T(kx), T(ky), T(kz)};
+    cplx<T> r[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) r[d] = c[d * total + t];
+    const cplx<T> div = mk<T>((kk[0] * r[0].x + kk[1] * r[1].x + kk[2] * r[2].x) * ikk,
+                              (kk[0] * r[0].y + kk[1] * r[1].y + kk[2] * r[2].y) * ikk);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      mu[d * total + t] = mk<T>(r[d].x - kk[d] * div.x, r[d].y - kk[d] * div.y);
+  }
+}
+
 // y = a + s x over whole buffers (n complex elements)
 template <typename T>
 __global__ void ns_axpy_kernel(const cplx<T>* a, const cplx<T>* x, cplx<T>* y, double s, int64_t n) {
@@ -504,7 +573,16 @@ struct NsState {
   // lambda_y0, lambda_k, vjp output; physical lambda_adv
   void* adj[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   void* ladv = nullptr;
+  // the right-hand side on kept modes (null: the plan's transforms), its
+  // spectra: y0, the stage state, k1, k2, k3; of the adjoint: 4 stage states
+  // (the first is y0), mu, lambda, the cotangents of y0 and k, the VJP
+  std::unique_ptr<NsLines> lines;
+  dev::NsKept kept{};
+  void* kept_rk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  void* kept_adj[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   ~NsState() {
+    for (auto p : kept_rk) cudaFree(p);
+    for (auto p : kept_adj) cudaFree(p);
     for (auto p : adj) cudaFree(p);
     cudaFree(ladv);
     for (auto p : dk) cudaFree(p);
@@ -523,6 +601,17 @@ void ck(cudaError_t e, const char* what) {
   if (e != cudaSuccess) fail(kErrCuda, std::string(what) + ": " + cudaGetErrorString(e));
 }
 }  // namespace
+
+// Work buffers of the right-hand side on the plan's transforms.
+static void ns_plan_alloc(NsState* s) {
+  const std::size_t rb = s->dbl ? 8 : 4, cb = 2 * rb;
+  for (auto& p : s->dk)
+    if (!p) ck(cudaMalloc(&p, s->nout * cb), "ns alloc");
+  for (auto& p : s->rk)
+    if (!p) ck(cudaMalloc(&p, s->nout * cb), "ns alloc");
+  for (auto& p : s->du)
+    if (!p) ck(cudaMalloc(&p, s->nin * rb), "ns alloc");
+}
 
 NsState* ns_create(const Plan* plan, double nu, double dt, double lx) {
   const auto& d = plan->desc();
@@ -552,9 +641,16 @@ NsState* ns_create(const Plan* plan, double nu, double dt, double lx) {
   s->nout = total_size(d.gout);
   const std::size_t rb = s->dbl ? 8 : 4, cb = 2 * rb;
   try {
-    for (auto& p : s->dk) ck(cudaMalloc(&p, s->nout * cb), "ns alloc");
-    for (auto& p : s->rk) ck(cudaMalloc(&p, s->nout * cb), "ns alloc");
-    for (auto& p : s->du) ck(cudaMalloc(&p, s->nin * rb), "ns alloc");
+    // (a compensated plan keeps its own transforms)
+    if (!d.comp)
+      s->lines = NsLines::create(s->dbl, s->g.nx, s->g.ny, s->g.nz, s->g.cx, s->g.cy, s->g.cz, s->g.kscale,
+                                 plan->scale(false), plan->scale(true));
+    if (s->lines) {
+      s->kept = dev::NsKept{2 * s->g.cx + 1, 2 * s->g.cy + 1, s->g.cz + 1};
+      for (auto& p : s->kept_rk) ck(cudaMalloc(&p, s->lines->elements() * cb), "ns alloc");
+    } else {
+      ns_plan_alloc(s);
+    }
     ck(cudaMalloc(&s->adv, s->nout * cb), "ns alloc");
     ck(cudaMalloc(&s->u, s->nin * rb), "ns alloc");
     ck(cudaMalloc(reinterpret_cast<void**>(&s->energy), sizeof(double)), "ns alloc");
@@ -649,6 +745,64 @@ static void ns_backward_phase(NsState* s, void* uk, cudaStream_t st) {
   }
 }
 
+// ---- on kept modes ----
+static void ns_gather(NsState* s, const void* uk, void* a, cudaStream_t st) {
+  using namespace dev;
+  const int64_t n = static_cast<int64_t>(s->kept.kx) * s->kept.ky * s->kept.kz;
+  if (s->dbl)
+    ns_gather_kernel<double><<<grid_of(n), 256, 0, st>>>(s->lout, static_cast<const double2*>(uk),
+                                                          static_cast<double2*>(a), s->g, s->kept);
+  else
+    ns_gather_kernel<float><<<grid_of(n), 256, 0, st>>>(s->lout, static_cast<const float2*>(uk),
+                                                         static_cast<float2*>(a), s->g, s->kept);
+  ck(cudaGetLastError(), "ns gather");
+}
+
+static void ns_scatter(NsState* s, const void* a, void* uk, cudaStream_t st) {
+  using namespace dev;
+  const int64_t n = static_cast<int64_t>(s->g.nx) * s->g.ny * s->g.nzh;
+  if (s->dbl)
+    ns_scatter_kernel<double><<<grid_of(n), 256, 0, st>>>(s->lout, static_cast<const double2*>(a),
+                                                           static_cast<double2*>(uk), s->g, s->kept);
+  else
+    ns_scatter_kernel<float><<<grid_of(n), 256, 0, st>>>(s->lout, static_cast<const float2*>(a),
+                                                          static_cast<float2*>(uk), s->g, s->kept);
+  ck(cudaGetLastError(), "ns scatter");
+}
+
+// the four RK4 stages on kept modes; the caller's spectrum is read at the
+// start and written (dealiased) at the end
+static void ns_kept_step(NsState* s, void* uk, cudaStream_t st) {
+  void *y0 = s->kept_rk[0], *state = s->kept_rk[1];
+  ns_gather(s, uk, y0, st);
+  NsLines::Update w;
+  w.out = state;
+  w.y0 = y0;
+  w.k1 = s->kept_rk[2];
+  w.k2 = s->kept_rk[3];
+  w.k3 = s->kept_rk[4];
+  w.nu = s->nu;
+  w.h = s->dt;
+  for (int step = 0; step < 4; ++step) {
+    w.u = step == 0 ? y0 : state;
+    w.step = step;
+    s->lines->rhs(w, st);
+  }
+  ns_scatter(s, state, uk, st);
+}
+
+// f(D uk) into dukdt; uk is left dealiased, as the reference's right-hand side does
+static void ns_kept_rhs(NsState* s, void* uk, void* dukdt, cudaStream_t st) {
+  ns_gather(s, uk, s->kept_rk[0], st);
+  NsLines::Update w;
+  w.u = s->kept_rk[0];
+  w.out = s->kept_rk[1];
+  w.nu = s->nu;
+  s->lines->rhs(w, st);
+  ns_scatter(s, s->kept_rk[1], dukdt, st);
+  ns_scatter(s, s->kept_rk[0], uk, st);
+}
+
 // step in 0..3: RK4 stage; step = -1: only the right-hand side, into `out`
 static void ns_rhs_stage(NsState* s, void* uk, int step, void* out, cudaStream_t st) {
   ns_backward_phase(s, uk, st);
@@ -684,6 +838,12 @@ void ns_batch_step(NsState* const* s, void* const* uks, int n, const Batch& batc
     for (int f : order) phase(f, batch.lane(st, lane_of[f]));
     batch.join(st, lanes);
   };
+  // kernels on kept modes are not batched: each field runs its whole step on
+  // its lane
+  if (std::any_of(s, s + n, [](const NsState* f) { return f->lines != nullptr; })) {
+    per_field([&](int f, cudaStream_t ls) { ns_step(s[f], uks[f], ls); });
+    return;
+  }
   for (int step = 0; step < 4; ++step) {
     per_field([&](int f, cudaStream_t ls) { ns_prep_phase(s[f], uks[f], ls); });
     for (int f = 0; f < n; ++f) {
@@ -710,9 +870,18 @@ void ns_batch_step(NsState* const* s, void* const* uks, int n, const Batch& batc
 
 const Plan* ns_plan(const NsState* s) { return s->plan; }
 
-void ns_rhs(NsState* s, void* uk, void* dukdt, cudaStream_t st) { ns_rhs_stage(s, uk, -1, dukdt, st); }
+void ns_rhs(NsState* s, void* uk, void* dukdt, cudaStream_t st) {
+  if (s->lines)
+    ns_kept_rhs(s, uk, dukdt, st);
+  else
+    ns_rhs_stage(s, uk, -1, dukdt, st);
+}
 
 void ns_step(NsState* s, void* uk, cudaStream_t st) {
+  if (s->lines) {
+    ns_kept_step(s, uk, st);
+    return;
+  }
   for (int step = 0; step < 4; ++step) ns_rhs_stage(s, uk, step, nullptr, st);
 }
 
@@ -871,6 +1040,7 @@ NsDiag ns_write_diagnostics(NsState* s, const void* uk, const std::string& dir, 
 // ---- adjoints ----
 static void ns_adj_alloc(NsState* s) {
   if (s->ladv) return;
+  ns_plan_alloc(s);
   const std::size_t cb = (s->dbl ? 16 : 8) * s->nout, rb = (s->dbl ? 8 : 4) * s->nin;
   for (auto& p : s->adj) ck(cudaMalloc(&p, cb), "ns adjoint alloc");
   ck(cudaMalloc(&s->ladv, rb), "ns adjoint alloc");
@@ -975,7 +1145,79 @@ static void ns_step_adjoint_t(NsState* s, const void* uk, void* lam, cudaStream_
   launch_dealias<T>(s, ly0, lam, st);
 }
 
+// ---- adjoints on kept modes: only those of the cotangent matter (f dealiases
+// its argument and its advection, and the result is dealiased) ----
+static bool ns_kept_adjoint(NsState* s) {
+  if (!s->lines || !s->lines->adjoint_supported()) return false;
+  for (auto& p : s->kept_adj)
+    if (!p) ck(cudaMalloc(&p, s->lines->elements() * (s->dbl ? 16 : 8)), "ns adjoint alloc");
+  s->lines->adjoint_alloc();
+  return true;
+}
+
+template <typename T>
+static void ns_kept_vjp(NsState* s, const void* y, const void* c, void* out, cudaStream_t st) {
+  using namespace dev;
+  using C = cplx<T>;
+  void* mu = s->kept_adj[3];
+  const int64_t n = static_cast<int64_t>(s->kept.kx) * s->kept.ky * s->kept.kz;
+  ns_kept_project_kernel<T><<<grid_of(n), 256, 0, st>>>(static_cast<const C*>(c), static_cast<C*>(mu), s->g, s->kept);
+  ck(cudaGetLastError(), "ns vjp projection");
+  s->lines->vjp(y, mu, out, s->nu, st);
+}
+
+template <typename T>
+static void ns_kept_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cudaStream_t st) {
+  void *y = s->kept_rk[0], *c = s->kept_adj[4], *out = s->kept_adj[7];
+  ns_gather(s, uk, y, st);
+  ns_gather(s, lam, c, st);
+  ns_kept_vjp<T>(s, y, c, out, st);
+  ns_scatter(s, out, grad, st);
+}
+
+// As ns_step_adjoint_t, on kept modes: the stage states a_i = a_1 + up h f(a_{i-1})
+// come straight out of the right-hand side's last kernel.
+template <typename T>
+static void ns_kept_step_adjoint(NsState* s, const void* uk, void* lam, cudaStream_t st) {
+  const double h = s->dt;
+  const std::size_t n = s->lines->elements();
+  void* a[4] = {s->kept_rk[0], s->kept_adj[0], s->kept_adj[1], s->kept_adj[2]};
+  void *l = s->kept_adj[4], *ly0 = s->kept_adj[5], *lk = s->kept_adj[6], *g = s->kept_adj[7];
+  ns_gather(s, uk, a[0], st);
+  ns_gather(s, lam, l, st);
+  const double up[3] = {0.5, 0.5, 1.0};  // a2 = a1 + k1 / 2, a3 = a1 + k2 / 2, a4 = a1 + k3
+  NsLines::Update w;
+  w.y0 = a[0];
+  w.nu = s->nu;
+  w.step = 5;
+  for (int i = 1; i < 4; ++i) {
+    w.u = a[i - 1];
+    w.out = a[i];
+    w.h = up[i - 1] * h;
+    s->lines->rhs(w, st);
+  }
+  const double direct[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};  // d S / d k_i
+  launch_axpy<T>(l, l, lk, direct[3] - 1.0, n, st);
+  for (int i = 3; i >= 0; --i) {
+    // g = f'(a_i)^T lk
+    ns_kept_vjp<T>(s, a[i], lk, g, st);
+    launch_axpy<T>(i == 3 ? l : ly0, g, ly0, h, n, st);
+    if (i > 0) {
+      launch_axpy<T>(l, l, lk, direct[i - 1] - 1.0, n, st);
+      launch_axpy<T>(lk, g, lk, h * up[i - 1], n, st);
+    }
+  }
+  ns_scatter(s, ly0, lam, st);
+}
+
 void ns_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cudaStream_t st) {
+  if (ns_kept_adjoint(s)) {
+    if (s->dbl)
+      ns_kept_rhs_adjoint<double>(s, uk, lam, grad, st);
+    else
+      ns_kept_rhs_adjoint<float>(s, uk, lam, grad, st);
+    return;
+  }
   if (s->dbl)
     ns_rhs_adjoint_t<double>(s, uk, lam, grad, st);
   else
@@ -983,6 +1225,13 @@ void ns_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cud
 }
 
 void ns_step_adjoint(NsState* s, const void* uk, void* lam, cudaStream_t st) {
+  if (ns_kept_adjoint(s)) {
+    if (s->dbl)
+      ns_kept_step_adjoint<double>(s, uk, lam, st);
+    else
+      ns_kept_step_adjoint<float>(s, uk, lam, st);
+    return;
+  }
   if (s->dbl)
     ns_step_adjoint_t<double>(s, uk, lam, st);
   else
