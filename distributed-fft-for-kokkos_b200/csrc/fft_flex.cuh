@@ -12,9 +12,9 @@
 //
 // Measured (B200, forward + backward; before: the table-driven kernel of
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
-// kernels): 300 x 250 x 360 complex64 3818 -> 593 us, 200 x 180 x 252 R2C / C2R
-// double 1633 -> 213 us, 131 x 105 x 157 R2C / C2R double 766 -> 187 us, 256^3
-// complex128 644 -> 558 us, 384^3 R2C / C2R double 1568 -> 1158 us.  On 2^k and
+// kernels): 300 x 250 x 360 complex64 3818 -> 555 us, 200 x 180 x 252 R2C / C2R
+// double 1633 -> 213 us, 131 x 105 x 157 R2C / C2R double 766 -> 174 us, 256^3
+// complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1158 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
 //
@@ -52,15 +52,18 @@ constexpr int resident_threads(int r, bool more) {
   if (sizeof(T) == 4)
     return more ? (r <= 12 ? 896 : r <= 16 ? 768 : r <= 21 ? 576 : 512)
                 : (r <= 8 ? 1280 : r <= 12 ? 1024 : r <= 16 ? 896 : r <= 21 ? 640 : r <= 25 ? 576 : 512);
-  return more ? (r <= 8 ? 768 : r <= 10 ? 640 : r <= 12 ? 512 : r <= 16 ? 448 : r <= 21 ? 320 : r <= 25 ? 288 : 256)
+  return more ? (r <= 8 ? 768 : r <= 10 ? 640 : r <= 12 ? 512 : r <= 16 ? 512 : r <= 21 ? 384 : r <= 25 ? 320 : 256)
               : (r <= 8 ? 896 : r <= 10 ? 768 : r <= 12 ? 640 : r <= 16 ? 512 : r <= 21 ? 448 : r <= 25 ? 384 : 256);
 }
 
-// Lines per tile: b-fast rows of at least 128 bytes; about 128 threads.
+// Lines per tile: about 128 threads.  b-fast rows of 128 bytes; of 64 bytes for
+// complex64 lines with R1 >= 12, whose 128-byte tiles are CTAs of 200 to 400
+// threads that spend their time at the barrier (300 x 250 x 360: stages of 104
+// and 103 us with 16 lines, 97 and 86 us with 8).
 template <typename T>
 constexpr int tile_lines(bool afast, int r) {
   if (afast) return 128 / r > 1 ? 128 / r : 1;
-  int b = sizeof(T) == 4 ? 16 : 8;
+  int b = sizeof(T) == 4 && r < 12 ? 16 : 8;
   while (b * r < 64) b *= 2;
   return b;
 }

@@ -21,7 +21,7 @@
 // The adjoint runs the transposes of the same steps.
 // Measured (B200; before: four backward transforms and one forward of the plan
 // around pointwise kernels): physical field to physical field over one RK4
-// step, 192^3 FP32 4172 -> 1904 us; step and gradient, 96^3 FP64 4748 -> 1656 us.
+// step, 192^3 FP32 4172 -> 1666 us; step and gradient, 96^3 FP64 4748 -> 1396 us.
 //
 // Each kernel is two passes of register codelets around one exchange, a kernel
 // per length (as in fft_flex.cuh).  Inverse transforms take the forward
@@ -188,6 +188,10 @@ __global__ void __launch_bounds__((LineShape<T, R1, R2>::NT), (LineShape<T, R1, 
 // back; lambda_u = sum_j lambda_j d_a u_j and h_a,j = u_a lambda_j forward
 // (weight 2 on the interior modes); W = lambda_u^ - i k_z h_z^ over field A,
 // h_y^ over B, h_x^ over C.
+// Every spectrum element is read once, scaled, and put to both positions of its
+// line that it makes; codelets that loaded their positions themselves read
+// each element twice with index and sign choices per position (192^3 FP32: 221
+// us a launch, 163 us this way).
 template <typename T>
 struct ZArgs {
   Grid g;
@@ -234,42 +238,46 @@ __global__ void __launch_bounds__((ZShape<T, R1, R2, ADJ>::NT), (ZShape<T, R1, R
   const int npair = min(S::G, (a.points + 1) / 2 - pair0);
   const C zero = mk<T>(T(0), T(0));
 
-  // back, pass 1: line = pair * NB + field * 3 + component
-  for (int it = threadIdx.x; it < npair * NB * R2; it += NT) {
-    const int line = it / R2, j = it % R2;
-    const int pr = line / NB, l = line % NB;
-    const int w = l / 3, d = l % 3;  // field 0 A, 1 B, 2 C, 3 D (= i k_z A), 4 lambda
+  // assemble: Z = X0 + i X1 of every line from the kept modes of the two
+  // points, scaled, in natural order (the cut positions are not written);
+  // line = pair * NB + field * 3 + component, field 0 A, 1 B, 2 C, 3 D = i k_z A,
+  // 4 lambda
+  constexpr int NI = ADJ ? 12 : 9;  // lines read: A, B, C (and lambda)
+  for (int it = threadIdx.x; it < npair * NI * kz; it += NT) {
+    int ln, m;
+    split_kz(a.g, it, &ln, &m);
+    const int pr = ln / NI, l = ln % NI;
     const int64_t pt = 2 * static_cast<int64_t>(pair0 + pr);
     const bool two = pt + 1 < a.points;
-    const C* x0 = (ADJ && w == 4 ? a.lambda + static_cast<int64_t>(d) * a.points * kz
-                                 : a.f + static_cast<int64_t>((w == 3 ? 0 : w) * 3 + d) * a.points * kz) + pt * kz;
-    const C* x1 = two ? x0 + kz : x0;
-    const T ks = T(a.g.kscale), ls = T(0.5 * a.lscale);
+    const C* x0 = (ADJ && l >= 9 ? a.lambda + static_cast<int64_t>(l - 9) * a.points * kz
+                                 : a.f + static_cast<int64_t>(l) * a.points * kz) + pt * kz + m;
+    const T sc = ADJ && l >= 9 ? T((m == 0 ? 1.0 : 0.5) * a.lscale) : T(a.back);
+    const C c0 = cscale(x0[0], sc), c1 = two ? cscale(x0[kz], sc) : zero;
+    auto put = [&](int line, C p, C q) {
+      C* o = s1 + (pr * NB + line) * P;
+      if (m == 0) {  // the imaginary part of the zero mode dropped
+        o[0] = mk<T>(p.x, q.x);
+      } else {
+        o[m] = mk<T>(p.x - q.y, p.y + q.x);
+        o[N - m] = mk<T>(p.x + q.y, q.x - p.y);
+      }
+    };
+    put(ADJ && l >= 9 ? l + 3 : l, c0, c1);
+    if (l < 3) {
+      const T k = T(m * a.g.kscale);
+      put(9 + l, ik<T>(k, c0), ik<T>(k, c1));
+    }
+  }
+  __syncthreads();
+  // back, pass 1
+  for (int it = threadIdx.x; it < npair * NB * R2; it += NT) {
+    const int line = it / R2, j = it % R2;
+    const C* b = s1 + line * P + j;
     C v[R1];
 #pragma unroll
     for (int r = 0; r < R1; ++r) {
       const int p = j + r * R2;
-      const bool mirror = 2 * p > N;
-      const int m = mirror ? N - p : p;
-      v[r] = zero;
-      if (m <= c) {
-        C c0 = x0[m], c1 = two ? x1[m] : zero;
-        if (w == 3) {
-          const T k = T(m) * ks;
-          c0 = ik<T>(k, c0);
-          c1 = ik<T>(k, c1);
-        }
-        if (ADJ && w == 4) {
-          const T sc = m == 0 ? T(2) * ls : ls;
-          c0 = cscale(c0, sc);
-          c1 = cscale(c1, sc);
-        }
-        // Z = X0 + i X1, the imaginary part of the zero mode dropped
-        if (r == 0 && m == 0)
-          v[r] = mk<T>(c0.x, c1.x);
-        else
-          v[r] = mirror ? mk<T>(c0.x + c1.y, c1.x - c0.y) : mk<T>(c0.x - c1.y, c0.y + c1.x);
-      }
+      v[r] = static_cast<unsigned>(p - c - 1) < static_cast<unsigned>(N - 2 * c - 1) ? zero : b[r * R2];
     }
     Dft<T, R1>::run(v);
     C* o = s0 + line * P + j * row;
@@ -277,18 +285,17 @@ __global__ void __launch_bounds__((ZShape<T, R1, R2, ADJ>::NT), (ZShape<T, R1, R
     for (int r = 0; r < R1; ++r) o[r] = v[r];
   }
   __syncthreads();
-  // back, pass 2: points in natural order, scaled (lambda carries its scale)
+  // back, pass 2: points in natural order
   for (int it = threadIdx.x; it < npair * NB * R1; it += NT) {
     const int line = it / R1, j = it % R1;
     C u[R2];
     flex::load_column<T, R2, R1, row>(s0 + line * P + j, tw, j, u);
     Dft<T, R2>::run(u);
-    const T sc = ADJ && line % NB >= 12 ? T(1) : T(a.back);
     C* o = s1 + line * P;
-    o[j == 0 ? 0 : N - j] = cscale(u[0], sc);
+    o[j == 0 ? 0 : N - j] = u[0];
     o += N - j;
 #pragma unroll
-    for (int r = 1; r < R2; ++r) o[-r * R1] = cscale(u[r], sc);
+    for (int r = 1; r < R2; ++r) o[-r * R1] = u[r];
   }
   __syncthreads();
   // products at the points: s1 (12 or 15 lines a pair) -> s0 (3 or 12 lines)
