@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(N / Vals<N>::value * B,
                                   (MinBlocks<T, N, N / Vals<N>::value * B, AFAST, AFF>::value))
     fft_fast_kernel(const StageArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  release_dependents();
   // grid (tiles_b, Eo0, Eo1): tile along b, coordinates along o0 and o1
   fast_tile<T, INV, N, B, AFAST, AFF>(A, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(N / Vals<N>::value * B,
 template <typename T, bool C2R, int N, int B, bool AFF>
 __global__ void __launch_bounds__(N / Vals<N>::value * B) fft_real_kernel(const StageArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  release_dependents();
   // grid (tiles_b, Eo0, Eo1): tile along b, coordinates along o0 and o1
   real_tile<T, C2R, N, B, AFF>(A, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
@@ -68,8 +70,7 @@ inline cudaError_t launch_fast_b(const StageArgs& A, cudaStream_t st) {
   auto k = fft_fast_kernel<T, INV, N, B, AF, AFF>;
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
-  k<<<fast_grid(A), N / Vals<N>::value * B, smem, st>>>(with_table_offsets(A));
-  return cudaGetLastError();
+  return launch_kernel_early(early_start(A, sizeof(cplx<T>)), k, fast_grid(A), N / Vals<N>::value * B, smem, st, with_table_offsets(A));
 }
 
 template <typename T, int N, bool C2R, int B, bool AFF = false>
@@ -79,8 +80,7 @@ inline cudaError_t launch_real_b(const StageArgs& A, cudaStream_t st) {
   auto k = fft_real_kernel<T, C2R, N, B, AFF>;
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
-  k<<<fast_grid(A), N / Vals<N>::value * B, smem, st>>>(with_table_offsets(A));
-  return cudaGetLastError();
+  return launch_kernel_early(early_start(A, sizeof(cplx<T>)), k, fast_grid(A), N / Vals<N>::value * B, smem, st, with_table_offsets(A));
 }
 
 // Launch of a general-layout stage (affine lines, axis-table sides or a

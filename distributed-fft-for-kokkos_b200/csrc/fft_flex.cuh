@@ -192,6 +192,7 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
   constexpr int B = S::B, M = S::m;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const s = reinterpret_cast<C*>(smem_raw);
+  release_dependents();
   const int t = threadIdx.x;
   const int per = kReal ? 2 * B : B;
   const int b0 = static_cast<int>(blockIdx.x) * per, nb = min(per, A.Eb - b0);
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
   const bool act1 = (AFAST ? t < B * R1 : j1 < R1) && line1 < nact;
 
   // ---- pass 1: codelets over positions j + r R2, row j of the matrix
+  dependency_wait();
   if (act2) {
     C v[R1];
     if constexpr (KIND == kR2C) {
@@ -402,8 +404,7 @@ cudaError_t launch_kernel(const StageArgs& A, const FlexArgs& F, cudaStream_t st
   auto k = fft_flex_kernel<T, KIND, AFAST, R1, R2, CHIRP>;
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), S::smem);
   if (e != cudaSuccess) return e;
-  k<<<fast_grid(A), S::NT, S::smem, st>>>(with_table_offsets(A), F);
-  return cudaGetLastError();
+  return launch_kernel_early(early_start(A, sizeof(cplx<T>)), k, fast_grid(A), S::NT, S::smem, st, with_table_offsets(A), F);
 }
 
 // The kernels of one length: C2C a-fast and b-fast, R2C and C2R (a-fast).

@@ -36,6 +36,7 @@ template <bool INV, int N, int PB, bool AFAST, bool COMP = false, bool ATAB = fa
 __global__ void __launch_bounds__(N / 8 * PB, (PairMinBlocks<N / 8 * PB, COMP>::value))
     fft_pair_kernel(const StageArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  release_dependents();
   // grid (tiles_b, Eo0, Eo1)
   pair_tile<INV, N, PB, AFAST, COMP, ATAB>(A, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(N / 8 * PB, 1) fft_pair_stream_kernel(const St
   using SH = SmemShape<double, N, PB, AFAST>;
   constexpr int LP = SH::LP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  release_dependents();
   C* tw = reinterpret_cast<C*>(smem_raw);
   float4* tile = reinterpret_cast<float4*>(smem_raw + sizeof(C) * N);
   const DevLayout ls = A.src, ld = A.dst;
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(N / 8 * PB, 1) fft_pair_stream_kernel(const St
   const C* in = reinterpret_cast<const C*>(A.in);
   C* out = reinterpret_cast<C*>(A.out);
 
+  dependency_wait();
   C v0[V], v1[V], w0[V], w1[V];
   int b0 = first * 2 * PB;
   int nb = min(2 * PB, A.Eb - b0);
@@ -116,8 +119,7 @@ static cudaError_t launch_pair_b(const StageArgs& A, cudaStream_t st) {
     auto k = fft_pair_kernel<INV, N, PB, AF, COMP, ATAB>;
     const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
-    k<<<fast_grid(A), N / 8 * PB, smem, st>>>(with_table_offsets(A));
-    return cudaGetLastError();
+    return launch_kernel_early(early_start(A, sizeof(float2)), k, fast_grid(A), N / 8 * PB, smem, st, with_table_offsets(A));
   }
 }
 
@@ -132,8 +134,7 @@ static cudaError_t launch_pair_stream(const StageArgs& A, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const dim3 grid(static_cast<unsigned>((A.tiles_b + A.tpc - 1) / A.tpc), static_cast<unsigned>(A.Eo0),
                   static_cast<unsigned>(A.Eo1));
-  k<<<grid, N / 8 * PB, smem, st>>>(with_table_offsets(A));
-  return cudaGetLastError();
+  return launch_kernel_early(early_start(A, sizeof(float2)), k, grid, N / 8 * PB, smem, st, with_table_offsets(A));
 }
 
 template <int N, bool INV, bool AF>

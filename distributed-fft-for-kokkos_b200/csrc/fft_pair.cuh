@@ -241,6 +241,7 @@ __device__ __forceinline__ void pair_tile(const StageArgs& A, int tb, int co0, i
     dof += __ldg(ld.t + A.d_to1 + co1);
   }
 
+  dependency_wait();
   C v0[V], v1[V];
   const C* in = reinterpret_cast<const C*>(A.in);
   load_pair<N, AFAST, ATAB>(A, in, so, b0, l0, l1, act0, act1, t, v0, v1);

@@ -72,6 +72,7 @@ __device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, i
     }
   }
 
+  dependency_wait();
   C v[V];
   constexpr int R0 = Radix<N, 0>::value, Q0 = V / R0;
   const C* in = reinterpret_cast<const C*>(A.in);
@@ -279,6 +280,7 @@ __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, i
   auto spos = [&](int p) -> int64_t { return satab ? __ldg(ls.t + A.s_ta + p) : p; };
   auto dpos = [&](int p) -> int64_t { return datab ? __ldg(ld.t + A.d_ta + p) : p; };
 
+  dependency_wait();
   C v[V];
   constexpr int R0 = Radix<N, 0>::value, Q0 = V / R0;
   if constexpr (!C2R) {

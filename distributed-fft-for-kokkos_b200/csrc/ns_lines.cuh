@@ -90,7 +90,7 @@ struct LineShape {
   static constexpr int B = flex::tile_lines<T>(false, R1);
   static constexpr size_t smem = sizeof(cplx<T>) * B * R1 * R2;
   static constexpr int NT = (B * R1 + 31) / 32 * 32;
-  static constexpr int fit = flex::resident_threads<T>(R1, true) / NT;
+  static constexpr int fit = (sizeof(T) == 4 && R1 <= 16 ? 896 : flex::resident_threads<T>(R1, true)) / NT;
   static constexpr int blocks = fit > 0 ? fit : 1;
 };
 
@@ -103,6 +103,7 @@ __global__ void __launch_bounds__((LineShape<T, R1, R2>::NT), (LineShape<T, R1, 
   constexpr bool kInverse = KIND == kXInverse || KIND == kYInverse;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const s = reinterpret_cast<C*>(smem_raw);
+  release_dependents();
   const Axis& ax = kX ? a.g.x : a.g.y;
   const int line = threadIdx.x % B, j = threadIdx.x / B;
   const int q = static_cast<int>(blockIdx.x) * B + line, d = blockIdx.y, f = blockIdx.z;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__((LineShape<T, R1, R2>::NT), (LineShape<T, R1, 
     points = (static_cast<int64_t>(fp * 3 + d) * a.g.x.n + first) * ax.n * kz + second;
     modes = (static_cast<int64_t>(fm * 3 + d) * a.g.x.n + first) * ax.k * kz + second;
   }
+  dependency_wait();
   if (live && j < R2) {
     C v[R1];
     if (kInverse) {
@@ -213,7 +215,7 @@ struct ZShape {
   static constexpr int NT = items <= 256 ? items : (items / 2 + 31) / 32 * 32 <= 256 ? (items / 2 + 31) / 32 * 32 : 256;
   static constexpr size_t smem = 2 * sizeof(cplx<T>) * G * back * P;
   static constexpr bool ok = smem <= 227 * 1024;
-  static constexpr int fit = flex::resident_threads<T>(R1, true) / NT;
+  static constexpr int fit = (sizeof(T) == 4 && R1 <= 16 ? 960 : flex::resident_threads<T>(R1, true)) / NT;
   static constexpr int blocks = fit > 0 ? fit : 1;
 };
 
@@ -229,6 +231,7 @@ __global__ void __launch_bounds__((ZShape<T, R1, R2, ADJ>::NT), (ZShape<T, R1, R
   using S = ZShape<T, R1, R2, ADJ>;
   constexpr int NB = S::back, NF = S::fwd, N = S::N, P = S::P, NT = S::NT, row = S::odd1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  release_dependents();
   C* const s0 = reinterpret_cast<C*>(smem_raw);
   C* const s1 = s0 + S::G * NB * P;
   const Axis& z = a.g.z;
@@ -237,6 +240,7 @@ __global__ void __launch_bounds__((ZShape<T, R1, R2, ADJ>::NT), (ZShape<T, R1, R
   const int pair0 = static_cast<int>(blockIdx.x) * S::G;
   const int npair = min(S::G, (a.points + 1) / 2 - pair0);
   const C zero = mk<T>(T(0), T(0));
+  dependency_wait();
 
   // assemble: Z = X0 + i X1 of every line from the kept modes of the two
   // points, scaled, in natural order (the cut positions are not written);

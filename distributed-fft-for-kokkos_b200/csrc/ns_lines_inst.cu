@@ -17,8 +17,8 @@ cudaError_t launch_line(const LineArgs<T>& a, int nf, cudaStream_t st) {
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), S::smem);
   if (e != cudaSuccess) return e;
   const dim3 grid(static_cast<unsigned>((a.lines + S::B - 1) / S::B), 3, static_cast<unsigned>(nf));
-  k<<<grid, S::NT, S::smem, st>>>(a);
-  return cudaGetLastError();
+  const size_t bytes = sizeof(cplx<T>) * R1 * R2 * a.lines * 3 * nf;
+  return launch_kernel_early(bytes <= kEarlyStartBytes, k, grid, S::NT, S::smem, st, a);
 }
 
 template <typename T, int R1, int R2, bool ADJ>
@@ -29,8 +29,9 @@ cudaError_t launch_z(const ZArgs<T>& a, cudaStream_t st) {
     const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), S::smem);
     if (e != cudaSuccess) return e;
     const int pairs = (a.points + 1) / 2;
-    k<<<static_cast<unsigned>((pairs + S::G - 1) / S::G), S::NT, S::smem, st>>>(a);
-    return cudaGetLastError();
+    const size_t bytes = sizeof(cplx<T>) * 9 * a.points * a.g.z.k;
+    return launch_kernel_early(bytes <= kEarlyStartBytes, k, dim3(static_cast<unsigned>((pairs + S::G - 1) / S::G)), S::NT,
+                               S::smem, st, a);
   } else {
     return cudaErrorInvalidValue;
   }
