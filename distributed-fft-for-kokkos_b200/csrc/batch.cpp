@@ -8,6 +8,7 @@
 #include <set>
 #include <string>
 #include <tuple>
+#include <utility>
 
 namespace dfft {
 
@@ -99,13 +100,43 @@ std::size_t Batch::launches(bool forward) const {
   return n;
 }
 
+// One group's launches of one stage, kMaxBatchFields fields each; the largest
+// fields come first, so that a launch ends with small tiles.
+void Batch::launch_group(const Group& g, cudaStream_t st) const {
+  auto tiles_of = [](const dev::StageArgs& A) { return static_cast<long long>(A.tiles_b) * A.Eo0 * A.Eo1; };
+  auto list = g.args;
+  std::stable_sort(list.begin(), list.end(),
+                   [&](const dev::StageArgs& x, const dev::StageArgs& y) { return tiles_of(x) > tiles_of(y); });
+  for (std::size_t c = 0; c < list.size(); c += dev::kMaxBatchFields) {
+    dev::BatchParams P;
+    std::memset(&P, 0, sizeof(P));
+    P.nfields = static_cast<int>(std::min<std::size_t>(dev::kMaxBatchFields, list.size() - c));
+    P.prefix[0] = 0;
+    for (int i = 0; i < P.nfields; ++i) {
+      P.f[i] = list[c + i];
+      const long long tiles = tiles_of(P.f[i]);
+      if (tiles >= (1ll << 31)) fail(kErrUnsupported, "too many tiles in one field of a batch");
+      P.prefix[i + 1] = P.prefix[i] + tiles;
+    }
+    const cudaError_t e = g.pair ? dev::launch_fft_batch_pair(P, g.inverse, g.afast, st)
+                                 : dev::launch_fft_batch(P, dbl_, g.kind, g.inverse, g.afast, st);
+    if (e != cudaSuccess) fail(kErrCuda, std::string("batched stage launch failed: ") + cudaGetErrorString(e));
+  }
+}
+
 void Batch::execute(const void* const* ins, void* const* outs, bool forward, cudaStream_t st) const {
   if (!ins || !outs) fail(kErrInvalidArgument, "null buffer arrays");
   for (std::size_t f = 0; f < plans_.size(); ++f) plans_[f]->check_buffers(ins[f], outs[f], forward);
   std::size_t nst = 0;
   for (const Plan* p : plans_) nst = std::max(nst, p->program(forward).size());
+  // the groups of every stage index, the stages that launch per field, and the
+  // group each field is in (numbered by their first field)
+  std::vector<std::vector<Group>> groups(nst);
+  std::vector<std::vector<std::pair<std::size_t, dev::StageArgs>>> single(nst);  // (field, args)
+  std::vector<std::vector<int>> member(nst);
   for (std::size_t s = 0; s < nst; ++s) {
-    std::map<GroupKey, std::vector<dev::StageArgs>> groups;
+    std::map<GroupKey, int> index;
+    member[s].assign(plans_.size(), -1);
     for (std::size_t f = 0; f < plans_.size(); ++f) {
       const Plan* p = plans_[f];
       const auto& prog = p->program(forward);
@@ -116,8 +147,7 @@ void Batch::execute(const void* const* ins, void* const* outs, bool forward, cud
       A.in = op.src == kBufIn ? const_cast<void*>(ins[f]) : op.src == kBufOut ? outs[f] : p->device_buffer(op.src);
       A.out = op.dst == kBufIn ? const_cast<void*>(ins[f]) : op.dst == kBufOut ? outs[f] : p->device_buffer(op.dst);
       if (!batchable(op)) {
-        const cudaError_t e = p->launch_op(op, A, st);
-        if (e != cudaSuccess) fail(kErrCuda, std::string("kernel launch failed: ") + cudaGetErrorString(e));
+        single[s].emplace_back(f, A);
         continue;
       }
       // the batched tile bodies: two lines per thread where the one-tile
@@ -128,42 +158,43 @@ void Batch::execute(const void* const* ins, void* const* outs, bool forward, cud
       const bool pair = pair_batchable(op, dbl_) && (A.load_afast || aligned);
       A.pairs = 0;
       A.comp = 0;
-      A.B = pair ? dev::batch_pair_lines(A.n, A.load_afast != 0) : dev::batch_stage_lines(A.n);
+      A.B = pair ? dev::batch_pair_lines(A.n, A.load_afast != 0) : dev::batch_stage_lines(dbl_, A.n);
       const int per = (op.kind == dev::kC2C) ? A.B : 2 * A.B;
       A.tiles_b = (A.Eb + per - 1) / per;
-      groups[GroupKey(op.kind, op.inverse, A.load_afast != 0, A.n, pair)].push_back(A);
-    }
-    // one launch per group (and per kMaxBatchFields fields of it); within a
-    // launch the largest fields come first, so the last work items the
-    // persistent CTAs pick up are small tiles and the launch ends evenly
-    int nl = 0;
-    for (auto& g : groups) nl += static_cast<int>((g.second.size() + dev::kMaxBatchFields - 1) / dev::kMaxBatchFields);
-    fork(st, nl);
-    auto tiles_of = [](const dev::StageArgs& A) { return static_cast<long long>(A.tiles_b) * A.Eo0 * A.Eo1; };
-    int li = 0;
-    for (auto& g : groups) {
-      auto list = g.second;
-      std::stable_sort(list.begin(), list.end(),
-                       [&](const dev::StageArgs& x, const dev::StageArgs& y) { return tiles_of(x) > tiles_of(y); });
-      for (std::size_t c = 0; c < list.size(); c += dev::kMaxBatchFields, ++li) {
-        dev::BatchParams P;
-        std::memset(&P, 0, sizeof(P));
-        P.nfields = static_cast<int>(std::min<std::size_t>(dev::kMaxBatchFields, list.size() - c));
-        P.prefix[0] = 0;
-        for (int i = 0; i < P.nfields; ++i) {
-          P.f[i] = list[c + i];
-          const long long tiles = tiles_of(P.f[i]);
-          if (tiles >= (1ll << 31)) fail(kErrUnsupported, "too many tiles in one field of a batch");
-          P.prefix[i + 1] = P.prefix[i] + tiles;
-        }
-        const cudaStream_t ls = lane(st, li);
-        const cudaError_t e = std::get<4>(g.first)
-                                  ? dev::launch_fft_batch_pair(P, std::get<1>(g.first), std::get<2>(g.first), ls)
-                                  : dev::launch_fft_batch(P, dbl_, std::get<0>(g.first), std::get<1>(g.first),
-                                                          std::get<2>(g.first), ls);
-        if (e != cudaSuccess) fail(kErrCuda, std::string("batched stage launch failed: ") + cudaGetErrorString(e));
+      const GroupKey key(op.kind, op.inverse, A.load_afast != 0, A.n, pair);
+      auto it = index.find(key);
+      if (it == index.end()) {
+        it = index.emplace(key, static_cast<int>(groups[s].size())).first;
+        groups[s].push_back(Group{op.kind, op.inverse, A.load_afast != 0, pair, {}});
       }
+      groups[s][it->second].args.push_back(A);
+      member[s][f] = it->second;
     }
+  }
+  // Fields that share a launch at one stage share it at every stage (cubic
+  // fields): each group's stages follow one another on a lane of their own,
+  // without waiting for the other groups between stages.  Else the groups of
+  // one stage run concurrently and join before the next.
+  bool chains = true;
+  for (std::size_t s = 0; s < nst; ++s)
+    chains = chains && single[s].empty() && member[s] == member[0];
+  if (chains && nst > 0) {
+    const int nl = static_cast<int>(groups[0].size());
+    fork(st, nl);
+    for (std::size_t s = 0; s < nst; ++s)
+      for (int g = 0; g < nl; ++g) launch_group(groups[s][g], lane(st, g));
+    join(st, nl);
+    return;
+  }
+  for (std::size_t s = 0; s < nst; ++s) {
+    for (auto& fa : single[s]) {
+      const Plan* p = plans_[fa.first];
+      const cudaError_t e = p->launch_op(p->program(forward)[s], fa.second, st);
+      if (e != cudaSuccess) fail(kErrCuda, std::string("kernel launch failed: ") + cudaGetErrorString(e));
+    }
+    const int nl = static_cast<int>(groups[s].size());
+    fork(st, nl);
+    for (int g = 0; g < nl; ++g) launch_group(groups[s][g], lane(st, g));
     join(st, nl);
   }
 }

@@ -1,5 +1,5 @@
 // Batched execution of many plans (fields of uneven sizes): every stage index
-// of the fused programs runs as one persistent launch per group of stages
+// of the fused programs runs as one launch per group of stages
 // that share kind, direction and row orientation (fft_batch.cu), instead of
 // one launch per field.
 #pragma once
@@ -27,7 +27,7 @@ class Batch {
   std::size_t size() const { return plans_.size(); }
   const std::vector<const Plan*>& plans() const { return plans_; }
 
-  // The launches of one stage index that belong to different groups touch
+  // Launches that belong to different groups touch
   // different fields: they run concurrently, forked from the caller's stream
   // onto kAux auxiliary streams and joined back (graph-capturable).  Callers
   // with per-field work of their own (the Navier-Stokes phases) use the same
@@ -38,6 +38,13 @@ class Batch {
   cudaStream_t lane(cudaStream_t st, int i) const { return i == 0 ? st : aux_[(i - 1) % kAux]; }
 
  private:
+  // fields that share a launch of one stage
+  struct Group {
+    int kind;
+    bool inverse, afast, pair;
+    std::vector<dev::StageArgs> args;
+  };
+  void launch_group(const Group& g, cudaStream_t st) const;
   std::vector<const Plan*> plans_;
   bool dbl_ = false;
   cudaStream_t aux_[kAux] = {};

@@ -150,11 +150,11 @@ int pair_tma_lines(int n);
 int pair_tma_line_options(int n, int* opts);
 cudaError_t launch_fft_pair_tma(const StageArgs& A, const void* map, const TmaCoords& T, bool inverse,
                                 cudaStream_t st);
-// Batched register stage (fft_batch.cu): one persistent launch runs the same
+// Batched register stage (fft_batch.cu): one launch runs the same
 // stage (kind, direction, row orientation) of up to kMaxBatchFields fields
 // of one line length; field f owns work items prefix[f] .. prefix[f+1] - 1,
 // its tiles (tb + tiles_b (co0 + Eo0 co1)).  Every field's StageArgs
-// must have B = batch_stage_lines(n) (complex lines per tile) and the tiles_b
+// must have B = batch_stage_lines(dbl, n) (complex lines per tile) and the tiles_b
 // that goes with it; the args are taken by value (kernel parameter space).
 constexpr int kMaxBatchFields = 48;
 // Two-line variant (fft_batch_sep.cu): complex64 C2C stages of 2^k points
@@ -167,7 +167,7 @@ struct BatchParams {
   StageArgs f[kMaxBatchFields];
 };
 bool batch_stage_supported(int n);
-int batch_stage_lines(int n);
+int batch_stage_lines(bool dbl, int n);
 // kind: kC2C, kR2C or kC2R (R2C / C2R: lines along a on both sides)
 cudaError_t launch_fft_batch(BatchParams& P, bool dbl, int kind, bool inverse, bool afast, cudaStream_t st);
 cudaError_t launch_fft_batch_pair(BatchParams& P, bool inverse, bool afast, cudaStream_t st);

@@ -1,15 +1,11 @@
-// Batched register FFT stages (sm_100a): one persistent launch runs one stage
-// of many fields of uneven sizes that share the stage's line length.
+// Batched register FFT stages (sm_100a): one launch runs one stage of many
+// fields of uneven sizes that share the stage's line length.
 //
-// A CTA of kBatchThreads threads walks work items blockIdx.x, +gridDim.x, ...
-// of a table that concatenates the tiles of every field; for each item it
-// finds the field (the item index only grows, so the field index only
-// advances), decodes the tile (tb, co0, co1) of that field's stage and runs
-// the tile body of the line length with B = kBatchThreads / (N / V) lines,
-// the same bodies as the one-tile-per-CTA kernels (fft_tile.cuh), at the
-// register budget of those kernels.  The twiddles are staged once per CTA; a
-// barrier separates consecutive tiles.  The host launches the lengths of one
-// stage index concurrently (batch.cpp).
+// The launch has a CTA per tile of every field; a CTA finds its field in the
+// prefix table of the kernel parameters, decodes the tile (tb, co0, co1) of
+// that field's stage and runs the tile body of the line length, the same
+// bodies as the one-field kernels (fft_tile.cuh) at their register budget.
+// The host launches the lengths of one stage index concurrently (batch.cpp).
 #include "fft_batch.cuh"
 
 namespace dfft {
@@ -36,10 +32,10 @@ bool batch_stage_supported(int n) {
   }
 }
 
-int batch_stage_lines(int n) {
+int batch_stage_lines(bool dbl, int n) {
   switch (n) {
 #define DFFT_LINES(N_) \
-  case N_: return BatchLines<N_>::value;
+  case N_: return dbl ? BatchLines<double, N_>::value : BatchLines<float, N_>::value;
     DFFT_BATCH_LENGTHS(DFFT_LINES)
 #undef DFFT_LINES
     default: return 0;

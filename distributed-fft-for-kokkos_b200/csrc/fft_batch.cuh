@@ -1,13 +1,13 @@
 // Kernels of the batched register stages (see fft_batch.cu): the tile bodies
-// of fft_tile.cuh behind a persistent work-table loop.  Instantiated for
+// of fft_tile.cuh behind a work table.  Instantiated for
 // general-layout sides (AFF, fft_batch.cu) and separable sides only
 // (fft_batch_sep.cu, fewer registers) in two translation units.
 #pragma once
 
 #include <cstring>
 
+#include "fft_fast.cuh"
 #include "fft_pair.cuh"
-#include "fft_tile.cuh"
 
 namespace dfft {
 namespace dev {
@@ -16,25 +16,19 @@ namespace batch {
 using namespace radix;
 
 
-constexpr int kBatchThreads = 256;
-
-// A launch covers the fields of one line length N, so each kernel carries one
-// tile body at a register budget of its own: resident threads per SM for
-// 8-value bodies 1536 complex64 / 768 complex128, for 24-value bodies 512 /
-// 256 (one step below the one-tile kernels of fft_fast.cu, which leaves the
-// work-table loop its registers without spilling); the general-layout
-// 8-value variant keeps the compiler's choice.
-template <typename T, int N, bool AFAST, bool AFF>
-struct BatchMinBlocks {
-  static constexpr bool v8 = Vals<N>::value == 8;
-  static constexpr int target = v8 ? (sizeof(T) == 4 ? 1536 : 768) : (sizeof(T) == 4 ? 512 : 256);
-  static constexpr int v = target / kBatchThreads;
-  static constexpr int value = (!(v8 && AFF) && v > 0) ? v : 1;
-};
-
-template <int N>
+// A launch covers the fields of one line length N, one tile per CTA, so each
+// kernel carries one tile body at the register budget of its one-field kernel
+// (MinBlocks of fft_fast.cuh).  Lines per tile: 256 threads for 8-value bodies;
+// 128 for 24-value ones where that leaves 128-byte rows (16 complex64 or 8
+// complex128), else 256.  (Persistent CTAs of 256 threads that walked the work
+// table held the 24-value bodies to 512 threads per SM, two CTAs waiting at
+// their barriers: 132 us a stage of five 192^3 complex64 fields.)
+template <typename T, int N>
 struct BatchLines {
-  static constexpr int value = kBatchThreads / (N / Vals<N>::value);
+  static constexpr int tt = N / Vals<N>::value;  // threads a line
+  static constexpr int rows = sizeof(T) == 4 ? 16 : 8;
+  static constexpr int threads = Vals<N>::value == 24 && rows * tt <= 128 ? 128 : 256;
+  static constexpr int value = threads / tt;
 };
 
 #define DFFT_BATCH_LENGTHS(X) \
@@ -50,40 +44,32 @@ __device__ __forceinline__ void decode(const StageArgs& A, unsigned local, int* 
   *co1 = static_cast<int>(rest / static_cast<unsigned>(A.Eo0));
 }
 
+// the field and tile of work item w: the fields of a launch follow one another
+__device__ __forceinline__ const StageArgs& locate(const BatchParams& P, long long w, int* tb, int* co0, int* co1) {
+  int f = 0;
+  while (w >= P.prefix[f + 1]) ++f;
+  decode(P.f[f], static_cast<unsigned>(w - P.prefix[f]), tb, co0, co1);
+  return P.f[f];
+}
+
 template <typename T, bool INV, bool AFAST, bool AFF, int N>
-__global__ void __launch_bounds__(kBatchThreads, (BatchMinBlocks<T, N, AFAST, AFF>::value))
+__global__ void __launch_bounds__((BatchLines<T, N>::threads), (MinBlocks<T, N, BatchLines<T, N>::threads, AFAST, AFF>::value))
     fft_batch_c2c_kernel(const __grid_constant__ BatchParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long total = P.prefix[P.nfields];
-  int f = 0;
-  bool first = true;  // the twiddles of N are staged by the CTA's first tile
-  for (long long w = blockIdx.x; w < total; w += gridDim.x) {
-    while (w >= P.prefix[f + 1]) ++f;
-    const StageArgs& A = P.f[f];
-    int tb, co0, co1;
-    decode(A, static_cast<unsigned>(w - P.prefix[f]), &tb, &co0, &co1);
-    fast_tile<T, INV, N, BatchLines<N>::value, AFAST, AFF>(A, tb, co0, co1, smem_raw, first);
-    first = false;
-    __syncthreads();  // the next tile restages its lines
-  }
+  release_dependents();
+  int tb, co0, co1;
+  const StageArgs& A = locate(P, blockIdx.x, &tb, &co0, &co1);
+  fast_tile<T, INV, N, BatchLines<T, N>::value, AFAST, AFF>(A, tb, co0, co1, smem_raw);
 }
 
 template <typename T, bool C2R, bool AFF, int N>
-__global__ void __launch_bounds__(kBatchThreads, (BatchMinBlocks<T, N, true, AFF>::value))
+__global__ void __launch_bounds__((BatchLines<T, N>::threads), (MinBlocks<T, N, BatchLines<T, N>::threads, true, AFF>::value))
     fft_batch_real_kernel(const __grid_constant__ BatchParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long total = P.prefix[P.nfields];
-  int f = 0;
-  bool first = true;
-  for (long long w = blockIdx.x; w < total; w += gridDim.x) {
-    while (w >= P.prefix[f + 1]) ++f;
-    const StageArgs& A = P.f[f];
-    int tb, co0, co1;
-    decode(A, static_cast<unsigned>(w - P.prefix[f]), &tb, &co0, &co1);
-    real_tile<T, C2R, N, BatchLines<N>::value, AFF>(A, tb, co0, co1, smem_raw, first);
-    first = false;
-    __syncthreads();
-  }
+  release_dependents();
+  int tb, co0, co1;
+  const StageArgs& A = locate(P, blockIdx.x, &tb, &co0, &co1);
+  real_tile<T, C2R, N, BatchLines<T, N>::value, AFF>(A, tb, co0, co1, smem_raw);
 }
 
 // Two-line (complex64, separable, 2^k points) batched C2C stage: the tile
@@ -100,18 +86,10 @@ template <bool INV, bool AFAST, int N>
 __global__ void __launch_bounds__(BatchPairs<N, AFAST>::threads, (BatchPairs<N, AFAST>::min_blocks))
     fft_batch_pair_kernel(const __grid_constant__ BatchParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long total = P.prefix[P.nfields];
-  int f = 0;
-  bool first = true;
-  for (long long w = blockIdx.x; w < total; w += gridDim.x) {
-    while (w >= P.prefix[f + 1]) ++f;
-    const StageArgs& A = P.f[f];
-    int tb, co0, co1;
-    decode(A, static_cast<unsigned>(w - P.prefix[f]), &tb, &co0, &co1);
-    pair_tile<INV, N, BatchPairs<N, AFAST>::value, AFAST>(A, tb, co0, co1, smem_raw, first);
-    first = false;
-    __syncthreads();
-  }
+  release_dependents();
+  int tb, co0, co1;
+  const StageArgs& A = locate(P, blockIdx.x, &tb, &co0, &co1);
+  pair_tile<INV, N, BatchPairs<N, AFAST>::value, AFAST>(A, tb, co0, co1, smem_raw);
 }
 
 template <typename T>
@@ -119,50 +97,44 @@ size_t tile_smem(int n, bool afast) {
   switch (n) {
 #define DFFT_SMEM(N_)                                                                                        \
   case N_:                                                                                                   \
-    return sizeof(cplx<T>) * (N_ + static_cast<size_t>(BatchLines<N_>::value) *                              \
-                                       (afast ? SmemShape<T, N_, BatchLines<N_>::value, true>::LP         \
-                                              : SmemShape<T, N_, BatchLines<N_>::value, false>::LP));
+    return sizeof(cplx<T>) * (N_ + static_cast<size_t>(BatchLines<T, N_>::value) *                              \
+                                       (afast ? SmemShape<T, N_, BatchLines<T, N_>::value, true>::LP         \
+                                              : SmemShape<T, N_, BatchLines<T, N_>::value, false>::LP));
     DFFT_BATCH_LENGTHS(DFFT_SMEM)
 #undef DFFT_SMEM
     default: return 0;
   }
 }
 
-template <int THREADS = kBatchThreads, typename K>
-cudaError_t launch_persistent(K kernel, BatchParams& P, size_t smem, cudaStream_t st) {
-  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
+template <int THREADS, typename K>
+cudaError_t launch_tiles(K kernel, const BatchParams& P, size_t smem, cudaStream_t st) {
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem)) != cudaSuccess)
-    return e;
-  long long grid = static_cast<long long>(sms) * (per_sm > 0 ? per_sm : 1);
   const long long total = P.prefix[P.nfields];
-  if (grid > total) grid = total;
-  if (grid < 1) return cudaSuccess;
-  kernel<<<static_cast<unsigned>(grid), THREADS, smem, st>>>(P);
-  return cudaGetLastError();
+  if (total < 1) return cudaSuccess;
+  if (total >= (1ll << 31)) return cudaErrorInvalidConfiguration;
+  return launch_kernel_early(true, kernel, dim3(static_cast<unsigned>(total)), THREADS, smem, st, P);
 }
 
 template <bool INV, bool AFAST, int N>
 cudaError_t launch_batch_pair_n(BatchParams& P, cudaStream_t st) {
   constexpr size_t smem = pair_tile_smem<N, BatchPairs<N, AFAST>::value, AFAST>();
   for (int i = 0; i < P.nfields; ++i) P.f[i] = with_table_offsets(P.f[i]);
-  return launch_persistent<BatchPairs<N, AFAST>::threads>(fft_batch_pair_kernel<INV, AFAST, N>, P, smem, st);
+  return launch_tiles<BatchPairs<N, AFAST>::threads>(fft_batch_pair_kernel<INV, AFAST, N>, P, smem, st);
 }
 
 template <typename T, bool AFF, int N>
 cudaError_t launch_batch_n(BatchParams& P, size_t smem, int kind, bool inverse, bool afast, cudaStream_t st) {
+  constexpr int NT = BatchLines<T, N>::threads;
   if (kind == kC2C) {
     if (inverse)
-      return afast ? launch_persistent(fft_batch_c2c_kernel<T, true, true, AFF, N>, P, smem, st)
-                   : launch_persistent(fft_batch_c2c_kernel<T, true, false, AFF, N>, P, smem, st);
-    return afast ? launch_persistent(fft_batch_c2c_kernel<T, false, true, AFF, N>, P, smem, st)
-                 : launch_persistent(fft_batch_c2c_kernel<T, false, false, AFF, N>, P, smem, st);
+      return afast ? launch_tiles<NT>(fft_batch_c2c_kernel<T, true, true, AFF, N>, P, smem, st)
+                   : launch_tiles<NT>(fft_batch_c2c_kernel<T, true, false, AFF, N>, P, smem, st);
+    return afast ? launch_tiles<NT>(fft_batch_c2c_kernel<T, false, true, AFF, N>, P, smem, st)
+                 : launch_tiles<NT>(fft_batch_c2c_kernel<T, false, false, AFF, N>, P, smem, st);
   }
-  if (kind == kR2C) return launch_persistent(fft_batch_real_kernel<T, false, AFF, N>, P, smem, st);
-  if (kind == kC2R) return launch_persistent(fft_batch_real_kernel<T, true, AFF, N>, P, smem, st);
+  if (kind == kR2C) return launch_tiles<NT>(fft_batch_real_kernel<T, false, AFF, N>, P, smem, st);
+  if (kind == kC2R) return launch_tiles<NT>(fft_batch_real_kernel<T, true, AFF, N>, P, smem, st);
   return cudaErrorInvalidValue;
 }
 

@@ -310,7 +310,7 @@ class Graph:
 
 class Batch:
     """Batched execution of distinct plans (fields of uneven sizes): one
-    persistent launch per stage of all fields.  ``execute(ins, outs,
+    launch per stage of all fields.  ``execute(ins, outs,
     direction)`` transforms ins[i] -> outs[i] with plans[i]."""
 
     def __init__(self, plans):

@@ -275,7 +275,7 @@ dfft_status dfft_graph_destroy(dfft_graph* graph);
  * plan twice is rejected: its scratch arrays would be shared).  One execute
  * transforms ins[i] -> outs[i] with plans[i] for every field, in the given
  * direction, on one stream: each stage index of the fields' programs runs as
- * one persistent launch per group of stages of the same kind, direction and
+ * one launch per group of stages of the same kind, direction and
  * row orientation (a work table of every field's tiles, any supported line
  * lengths: 2^k up to 2048 and 3 * 2^k up to 768, register kernels), instead
  * of one launch per field; stages outside that set launch per field.  Buffers
