@@ -194,7 +194,6 @@ Plan::Plan(const PlanDesc& d, bool on_device) : d_(d), on_device_(on_device) {
     if (d_err_) cudaFree(d_err_);
     for (auto& kv : blue_tables_)
       for (void* p : kv.second) cudaFree(p);
-    for (auto& kv : flex_tables_) cudaFree(kv.second);
     throw;
   }
 }
@@ -207,7 +206,6 @@ Plan::~Plan() {
   if (d_err_) cudaFree(d_err_);
   for (auto& kv : blue_tables_)
     for (void* p : kv.second) cudaFree(p);
-  for (auto& kv : flex_tables_) cudaFree(kv.second);
 }
 
 void Plan::analyze() {
@@ -392,24 +390,22 @@ std::vector<double> two_pass_twiddles(int r1, int r2) {
   return h;
 }
 
-const void* Plan::flex_twiddle(int r1, int r2) {
+// The table in the plan's precision, stored with the layout tables (one
+// upload): its offset there.
+std::int64_t Plan::flex_twiddle(int r1, int r2) {
   auto key = std::make_pair(r1, r2);
   auto it = flex_tables_.find(key);
   if (it != flex_tables_.end()) return it->second;
   const std::vector<double> h = two_pass_twiddles(r1, r2);
   const std::vector<float> hf(h.begin(), h.end());
-  void* p = nullptr;
   const std::size_t bytes = h.size() * (d_.dbl ? 8 : 4);
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    fail(kErrAlloc, "cudaMalloc of twiddle table failed");
-  }
-  flex_tables_[key] = p;
-  workspace_bytes_ += bytes;
-  cuda_check(cudaMemcpy(p, d_.dbl ? static_cast<const void*>(h.data()) : static_cast<const void*>(hf.data()), bytes,
-                        cudaMemcpyHostToDevice),
-             "twiddle upload");
-  return p;
+  if (host_tables_.size() % 2) host_tables_.push_back(0);  // 16-byte elements
+  const std::int64_t off = static_cast<std::int64_t>(host_tables_.size());
+  host_tables_.resize(host_tables_.size() + (bytes + 7) / 8);
+  std::memcpy(host_tables_.data() + off, d_.dbl ? static_cast<const void*>(h.data()) : static_cast<const void*>(hf.data()),
+              bytes);
+  flex_tables_[key] = off;
+  return off;
 }
 
 void Plan::select_flex(Op& op) const {
@@ -479,7 +475,7 @@ bool Plan::add_flex(Op& op) {
   op.fx = dev::FlexArgs{};
   op.fx.n = A.n;
   op.fx.m = m;
-  op.fx.tw = flex_twiddle(r1, r2);
+  op.fx_tw = flex_twiddle(r1, r2);  // resolved by allocate_device
   if (chirp)
     bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &op.fx.chirp, &op.fx.filter,
                      &op.fx.filter_inverse);
@@ -1067,7 +1063,6 @@ void Plan::build_adjoint(bool of_forward) {
   prog.clear();
   auto order = fft_axis_order();
   const std::size_t S = order.size();
-  const std::size_t ar = order.front();  // R2C axis
   Layout I;
   I.gext = d_.gout;
   I.topo.assign(d_.gout.size(), 1);
@@ -1399,6 +1394,7 @@ void Plan::allocate_device() {
         op.sa.src = dev_layout(op.src_layout);
         op.sa.dst = dev_layout(op.dst_layout);
         op.sa.err = d_err_;
+        if (op.flex) op.fx.tw = d_tables_ + op.fx_tw;
       } else if (op.type == Op::Pack || op.type == Op::All2All || op.type == Op::Unpack) {
         op.xa.geo = d_tables_ + reinterpret_cast<std::intptr_t>(op.xa.geo);
         if (op.type == Op::Pack) op.xa.lay = dev_layout(op.src_layout);

@@ -87,6 +87,7 @@ struct Op {
   // the tuner may pick; flex_B complex lines per tile
   bool flex = false;
   dev::FlexArgs fx{};
+  std::int64_t fx_tw = 0;  // its twiddles, in the plan's tables
   int flex_B = 0;
   TmaSource tma;      // source description of a TMA-eligible b-fast pair stage
   // chirp-z stage (line length with a prime factor above 13): make_stage marks
@@ -218,8 +219,8 @@ class Plan {
   std::map<std::pair<std::size_t, std::size_t>, std::vector<void*>> blue_tables_;  // (n, m) -> chirp, filter fwd / inv
   void bluestein_tables(std::size_t n, std::size_t m, const void** chirp, const void** ffwd, const void** finv);
   // Twiddles of an m = R1 R2 point two-pass stage (dev::FlexArgs::tw).
-  std::map<std::pair<int, int>, void*> flex_tables_;
-  const void* flex_twiddle(int r1, int r2);
+  std::map<std::pair<int, int>, std::int64_t> flex_tables_;
+  std::int64_t flex_twiddle(int r1, int r2);
   void select_flex(Op& op) const;
   bool add_flex(Op& op);
   std::int64_t add_geo(const Layout& L, const BlockInfo& b, std::size_t pc);
