@@ -58,6 +58,9 @@ struct StageArgs {
   // the two-pass kernel (fft_flex.cuh)
   int pairs;
   int tpc;
+  // 1: the layout tables are written by work before it in the stream, so the
+  // kernel must not start (and read them) early
+  int plain_launch;
   // device error word of the plan: kernels with bounded waits set it when a
   // wait runs out (1: a TMA tile load never completed)
   int* err;

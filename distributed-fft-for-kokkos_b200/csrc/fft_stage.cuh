@@ -66,7 +66,7 @@ inline cudaError_t launch_kernel_early(bool early, void (*kernel)(P...), dim3 gr
 
 // a stage's early start: by the bytes of the array it reads (complex elements)
 inline bool early_start(const StageArgs& A, size_t elem) {
-  return static_cast<size_t>(A.n) * A.Eb * A.Eo0 * A.Eo1 * elem <= kEarlyStartBytes;
+  return !A.plain_launch && static_cast<size_t>(A.n) * A.Eb * A.Eo0 * A.Eo1 * elem <= kEarlyStartBytes;
 }
 
 // Element offset of global coordinate c (nd axes) in a layout.

@@ -222,6 +222,7 @@ dfft_status dfft_noalloc_impl(const void* in, void* out, int64_t n0, int64_t n1,
     A.src_abase = A.dst_abase = 0;
     A.src_astride = A.dst_astride = (a == 0) ? n1 * n2 : (a == 1) ? n2 : 1;
     A.scale = si == 2 ? scale : 1.0;
+    A.plain_launch = 1;  // the tables are filled by the launch above
     A.tw = dbl ? static_cast<const void*>(s->tw64 + tw_offset(A.n))
                : static_cast<const void*>(s->tw32 + tw_offset(A.n));
     if (launch_fft_fast(A, dbl, !fwd, a == 2, cs) != cudaSuccess) {
