@@ -13,7 +13,7 @@
 // Measured (B200, forward + backward; before: the table-driven kernel of
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
 // kernels): 300 x 250 x 360 complex64 3818 -> 555 us, 200 x 180 x 252 R2C / C2R
-// double 1633 -> 213 us, 131 x 105 x 157 R2C / C2R double 766 -> 174 us, 256^3
+// double 1633 -> 213 us, 131 x 105 x 157 R2C / C2R double 766 -> 155 us, 256^3
 // complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1158 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
@@ -217,10 +217,35 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
   const bool act2 = (AFAST ? t < B * R2 : j2 < R2) && line2 < nact;
   const bool act1 = (AFAST ? t < B * R1 : j1 < R1) && line1 < nact;
 
-  // ---- pass 1: codelets over positions j + r R2, row j of the matrix
   dependency_wait();
+  if constexpr (KIND == kC2R && CHIRP) {
+    // Z = X0 + i X1 over the full line, from the two half spectra (imaginary
+    // parts of DC and Nyquist dropped), in natural order
+    constexpr int TPL = S::NT / B;  // threads a line
+    const int line = t / TPL;
+    if (line < nact) {
+      const bool two = 2 * line + 1 < nb;
+      const C* x0 = reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line, co0, co1).base;
+      const C* x1 = two ? reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line + 1, co0, co1).base : x0;
+      const T wt = T(A.weight);
+      for (int k = t % TPL; k <= n / 2; k += TPL) {
+        C c0 = x0[k];
+        C c1 = two ? x1[k] : mk<T>(T(0), T(0));
+        if (k == 0 || 2 * k == n) {
+          at(line, k) = mk<T>(c0.x, c1.x);
+        } else {
+          c0 = cscale(c0, wt);
+          c1 = cscale(c1, wt);
+          at(line, k) = mk<T>(c0.x - c1.y, c0.y + c1.x);
+          at(line, n - k) = mk<T>(c0.x + c1.y, c1.x - c0.y);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // ---- pass 1: codelets over positions j + r R2, row j of the matrix
+  C v[R1];
   if (act2) {
-    C v[R1];
     if constexpr (KIND == kR2C) {
       const T* in = reinterpret_cast<const T*>(A.in);
 #pragma unroll
@@ -230,28 +255,33 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
       if (2 * line2 + 1 < nb)
         positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + 2 * line2 + 1, co0, co1), j2, n,
                                         [&](int r, int64_t o) { v[r].y = in[o]; });
+    } else if constexpr (KIND == kC2R && CHIRP) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r)
+        v[r] = j2 + r * R2 < n ? at(line2, j2 + r * R2) : mk<T>(T(0), T(0));
     } else if constexpr (KIND == kC2R) {
-      // Z = X0 + i X1 over the full line, from the two half spectra
-      // (imaginary parts of DC and Nyquist dropped)
+      // Z from the half spectra directly, every mode loaded for both positions
+      // it makes: through shared memory as in the chirp-z form, with its
+      // barriers, 384^3 double took 273 us instead of 221 (131 x 105 x 157
+      // chirp-z lines, where the loads' index choices weigh more, 36 instead of
+      // 46)
       const bool two = 2 * line2 + 1 < nb;
       const C* x0 = reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2, co0, co1).base;
       const C* x1 = two ? reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2 + 1, co0, co1).base : x0;
+      const T wt = T(A.weight);
 #pragma unroll
       for (int r = 0; r < R1; ++r) {
         const int p = j2 + r * R2;
-        v[r] = mk<T>(T(0), T(0));
-        if (!CHIRP || p < n) {
-          const bool mirror = 2 * p > n;
-          const int q = mirror ? n - p : p;
-          C c0 = x0[q];
-          C c1 = two ? x1[q] : mk<T>(T(0), T(0));
-          if (q == 0 || 2 * q == n) {
-            v[r] = mk<T>(c0.x, c1.x);
-          } else {
-            c0 = cscale(c0, T(A.weight));
-            c1 = cscale(c1, T(A.weight));
-            v[r] = mirror ? mk<T>(c0.x + c1.y, c1.x - c0.y) : mk<T>(c0.x - c1.y, c0.y + c1.x);
-          }
+        const bool mirror = 2 * p > M;
+        const int q = mirror ? M - p : p;
+        C c0 = x0[q];
+        C c1 = two ? x1[q] : mk<T>(T(0), T(0));
+        if (q == 0 || 2 * q == M) {
+          v[r] = mk<T>(c0.x, c1.x);
+        } else {
+          c0 = cscale(c0, wt);
+          c1 = cscale(c1, wt);
+          v[r] = mirror ? mk<T>(c0.x + c1.y, c1.x - c0.y) : mk<T>(c0.x - c1.y, c0.y + c1.x);
         }
       }
     } else {
@@ -269,6 +299,9 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
         if (j2 + r * R2 < n) v[r] = cmul(v[r], chirp(j2 + r * R2));
     }
     Dft<T, R1>::run(v);
+  }
+  if constexpr (KIND == kC2R && CHIRP) __syncthreads();  // every position read: the buffer takes the matrices
+  if (act2) {
     C* o = &at(line2, j2 * row1);
 #pragma unroll
     for (int r = 0; r < R1; ++r) o[r * el] = v[r];

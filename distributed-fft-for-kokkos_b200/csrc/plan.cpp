@@ -1549,36 +1549,45 @@ void Plan::autotune() {
       for (int i = 0; i < nopt; ++i) cand.push_back(opts[i]);
       if (op.flex) cand.push_back(kFlexCode);
       int best = A.pairs == 4 ? kFlexCode : A.pairs == 3 ? kTmaCode + A.B : A.pairs == 2 ? kStreamCode + A.tpc : (A.pairs ? kPairCode : 0) + A.B;
-      float best_ms = std::numeric_limits<float>::max();
       cudaEvent_t e0, e1;
       cuda_check(cudaEventCreate(&e0), "tuner event");
       cuda_check(cudaEventCreate(&e1), "tuner event");
-      for (int code : cand) {
+      auto timed = [&](int code, int reps) {
         apply(code);
         dev::StageArgs T = A;
         T.in = t_in;
         T.out = t_out;
-        if (launch_stage(op, T, st) != cudaSuccess) {
-          cudaGetLastError();
-          continue;
-        }
-        auto timed = [&](int reps) {
-          cudaEventRecord(e0, st);
-          for (int r = 0; r < reps; ++r) launch_stage(op, T, st);
-          cudaEventRecord(e1, st);
-          cuda_check(cudaEventSynchronize(e1), "tuner sync");
-          float ms = 0.f;
-          cudaEventElapsedTime(&ms, e0, e1);
-          return ms / static_cast<float>(reps);
-        };
-        // short launches again: three of them measure the launch gaps too
-        float ms = timed(3);
-        if (ms < 0.05f) ms = std::min(timed(10), timed(10));
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = code;
-        }
+        cudaEventRecord(e0, st);
+        for (int r = 0; r < reps; ++r)
+          if (launch_stage(op, T, st) != cudaSuccess) {
+            cudaGetLastError();
+            return std::numeric_limits<float>::max();
+          }
+        cudaEventRecord(e1, st);
+        cuda_check(cudaEventSynchronize(e1), "tuner sync");
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        return ms / static_cast<float>(reps);
+      };
+      // every candidate over 3 launches (after one warm-up); short ones, whose
+      // launch gaps three launches measure too, again: the three fastest twice
+      // more over 10
+      std::vector<std::pair<float, int>> order;
+      for (int code : cand) {
+        if (timed(code, 1) == std::numeric_limits<float>::max()) continue;
+        order.emplace_back(timed(code, 3), code);
       }
+      std::stable_sort(order.begin(), order.end(),
+                       [](const std::pair<float, int>& x, const std::pair<float, int>& y) { return x.first < y.first; });
+      if (!order.empty() && order.front().first < 0.06f) {
+        if (order.size() > 3) order.resize(3);
+        for (auto& o : order) o.first = std::numeric_limits<float>::max();
+        for (int round = 0; round < 2 && order.size() > 1; ++round)
+          for (auto& o : order) o.first = std::min(o.first, timed(o.second, 10));
+        std::stable_sort(order.begin(), order.end(),
+                         [](const std::pair<float, int>& x, const std::pair<float, int>& y) { return x.first < y.first; });
+      }
+      if (!order.empty()) best = order.front().second;
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       apply(best);
