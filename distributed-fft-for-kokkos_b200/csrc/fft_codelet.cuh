@@ -303,17 +303,16 @@ struct DftOdd {
     for (int m = 0; m < H; ++m) v[0] = cadd(v[0], t[m]);
 #pragma unroll
     for (int q = 1; q <= H; ++q) {
-      C re = v0, im = mk<T>(T(0), T(0));
+      C re = v0, im;
 #pragma unroll
       for (int m = 1; m <= H; ++m) {
         const int e = (m * q) % R, f = e <= H ? e : R - e;
         const T c = T(Root<R>::c(f)), s = e <= H ? T(Root<R>::s(f)) : T(-Root<R>::s(f));
-        re = cadd(re, cscale(t[m - 1], c));
-        im = cadd(im, cscale(d[m - 1], s));
+        re = cfma(t[m - 1], c, re);
+        im = m == 1 ? cscale(d[0], s) : cfma(d[m - 1], s, im);
       }
-      const C r = rot<false>(im);
-      v[q] = cadd(re, r);
-      v[R - q] = csub(re, r);
+      v[q] = cadd_rot<false>(re, im);
+      v[R - q] = csub_rot<false>(re, im);
     }
   }
 };

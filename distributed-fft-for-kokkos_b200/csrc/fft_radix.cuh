@@ -14,12 +14,12 @@ namespace radix {
 
 template <bool INV, typename C>
 __device__ __forceinline__ void r4(C& v0, C& v1, C& v2, C& v3) {
-  C s02 = cadd(v0, v2), d02 = csub(v0, v2);
-  C s13 = cadd(v1, v3), d13 = rot<INV>(csub(v1, v3));
+  const C s02 = cadd(v0, v2), d02 = csub(v0, v2);
+  const C s13 = cadd(v1, v3), d13 = csub(v1, v3);
   v0 = cadd(s02, s13);
   v2 = csub(s02, s13);
-  v1 = cadd(d02, d13);
-  v3 = csub(d02, d13);
+  v1 = cadd_rot<INV>(d02, d13);
+  v3 = csub_rot<INV>(d02, d13);
 }
 
 template <typename T, bool INV>
@@ -30,23 +30,17 @@ __device__ __forceinline__ void r8(cplx<T>* v) {
   C o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
   r4<INV>(e0, e1, e2, e3);
   r4<INV>(o0, o1, o2, o3);
-  C t1, t3;
-  if (INV) {
-    t1 = mk<T>(h * (o1.x - o1.y), h * (o1.x + o1.y));
-    t3 = mk<T>(-h * (o3.x + o3.y), h * (o3.x - o3.y));
-  } else {
-    t1 = mk<T>(h * (o1.x + o1.y), h * (o1.y - o1.x));
-    t3 = mk<T>(h * (o3.y - o3.x), -h * (o3.x + o3.y));
-  }
-  C t2 = rot<INV>(o2);
+  // w^1 o1 = h u1, w^3 o3 = h u3
+  const C u1 = INV ? mk<T>(o1.x - o1.y, o1.x + o1.y) : mk<T>(o1.x + o1.y, o1.y - o1.x);
+  const C u3 = INV ? mk<T>(-o3.x - o3.y, o3.x - o3.y) : mk<T>(o3.y - o3.x, -o3.x - o3.y);
   v[0] = cadd(e0, o0);
   v[4] = csub(e0, o0);
-  v[1] = cadd(e1, t1);
-  v[5] = csub(e1, t1);
-  v[2] = cadd(e2, t2);
-  v[6] = csub(e2, t2);
-  v[3] = cadd(e3, t3);
-  v[7] = csub(e3, t3);
+  v[1] = cfma(u1, h, e1);
+  v[5] = cfma(u1, -h, e1);
+  v[2] = cadd_rot<INV>(e2, o2);
+  v[6] = csub_rot<INV>(e2, o2);
+  v[3] = cfma(u3, h, e3);
+  v[7] = cfma(u3, -h, e3);
 }
 
 template <typename T, bool INV>
@@ -54,11 +48,11 @@ __device__ __forceinline__ void r3(cplx<T>* v) {
   using C = cplx<T>;
   const T c3 = T(0.86602540378443864676372317075293618347);  // sqrt(3)/2
   const C t = cadd(v[1], v[2]);
-  const C d = rot<INV>(cscale(csub(v[1], v[2]), c3));
-  const C m = csub(v[0], cscale(t, T(0.5)));
+  const C d = csub(v[1], v[2]);
+  const C m = cfma(t, T(-0.5), v[0]);
   v[0] = cadd(v[0], t);
-  v[1] = cadd(m, d);
-  v[2] = csub(m, d);
+  v[1] = cfma_rot<INV>(d, c3, m);
+  v[2] = cfma_rot<INV>(d, -c3, m);
 }
 
 template <typename T, bool INV, int R>

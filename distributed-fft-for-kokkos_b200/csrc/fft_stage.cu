@@ -16,7 +16,7 @@
 #include <map>
 #include <mutex>
 
-#include "fft_stage.cuh"
+#include "fft_radix.cuh"
 
 namespace dfft {
 namespace dev {
@@ -24,56 +24,6 @@ namespace dev {
 // ---------------------------------------------------------------------------
 // Radix-R DFTs on registers.  Forward: X_q = sum_r v_r exp(-2 pi i r q / R).
 // ---------------------------------------------------------------------------
-template <bool INV, typename C>
-__device__ __forceinline__ void dft4(C& v0, C& v1, C& v2, C& v3) {
-  C s02 = cadd(v0, v2), d02 = csub(v0, v2);
-  C s13 = cadd(v1, v3), d13 = rot<INV>(csub(v1, v3));
-  v0 = cadd(s02, s13);
-  v2 = csub(s02, s13);
-  v1 = cadd(d02, d13);
-  v3 = csub(d02, d13);
-}
-
-template <typename T, bool INV>
-__device__ __forceinline__ void dft8(cplx<T>* v) {
-  using C = cplx<T>;
-  const T h = T(0.70710678118654752440084436210484903928);  // sqrt(1/2)
-  C e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-  C o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-  dft4<INV>(e0, e1, e2, e3);
-  dft4<INV>(o0, o1, o2, o3);
-  // w^1 o1, w^2 o2, w^3 o3 with w = exp(-/+ i pi / 4)
-  C t1, t3;
-  if (INV) {
-    t1 = mk<T>(h * (o1.x - o1.y), h * (o1.x + o1.y));
-    t3 = mk<T>(-h * (o3.x + o3.y), h * (o3.x - o3.y));
-  } else {
-    t1 = mk<T>(h * (o1.x + o1.y), h * (o1.y - o1.x));
-    t3 = mk<T>(h * (o3.y - o3.x), -h * (o3.x + o3.y));
-  }
-  C t2 = rot<INV>(o2);
-  v[0] = cadd(e0, o0);
-  v[4] = csub(e0, o0);
-  v[1] = cadd(e1, t1);
-  v[5] = csub(e1, t1);
-  v[2] = cadd(e2, t2);
-  v[6] = csub(e2, t2);
-  v[3] = cadd(e3, t3);
-  v[7] = csub(e3, t3);
-}
-
-template <typename T, bool INV>
-__device__ __forceinline__ void dft3(cplx<T>* v) {
-  using C = cplx<T>;
-  const T c3 = T(0.86602540378443864676372317075293618347);  // sqrt(3)/2
-  C t = cadd(v[1], v[2]);
-  C d = rot<INV>(cscale(csub(v[1], v[2]), c3));
-  C m = csub(v[0], cscale(t, T(0.5)));
-  v[0] = cadd(v[0], t);
-  v[1] = cadd(m, d);
-  v[2] = csub(m, d);
-}
-
 template <typename T, bool INV>
 __device__ __forceinline__ void dft5(cplx<T>* v) {
   using C = cplx<T>;
@@ -85,15 +35,15 @@ __device__ __forceinline__ void dft5(cplx<T>* v) {
   const T s2 = T(0.58778525229247312916870595463907276860);
   C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
   C d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
-  C a1 = cadd(v[0], cadd(cscale(t1, c1), cscale(t2, c2)));
-  C a2 = cadd(v[0], cadd(cscale(t1, c2), cscale(t2, c1)));
-  C b1 = rot<INV>(cadd(cscale(d1, s1), cscale(d2, s2)));
-  C b2 = rot<INV>(csub(cscale(d1, s2), cscale(d2, s1)));
+  const C a1 = cfma(t2, c2, cfma(t1, c1, v[0]));
+  const C a2 = cfma(t2, c1, cfma(t1, c2, v[0]));
+  const C b1 = cfma(d2, s2, cscale(d1, s1));
+  const C b2 = cfma(d2, -s1, cscale(d1, s2));
   v[0] = cadd(v[0], cadd(t1, t2));
-  v[1] = cadd(a1, b1);
-  v[4] = csub(a1, b1);
-  v[2] = cadd(a2, b2);
-  v[3] = csub(a2, b2);
+  v[1] = cadd_rot<INV>(a1, b1);
+  v[4] = csub_rot<INV>(a1, b1);
+  v[2] = cadd_rot<INV>(a2, b2);
+  v[3] = csub_rot<INV>(a2, b2);
 }
 
 // Odd radix R: pairwise form; cos and sin of 2 pi m / R are read from the
@@ -122,12 +72,11 @@ __device__ __forceinline__ void dft_odd(cplx<T>* v, const cplx<T>* tw, int n) {
     for (int m = 1; m <= H; ++m) {
       const int e = (m * q) % R;
       const C w = tw[e * step];  // (cos, -sin) of 2 pi e / R
-      re = cadd(re, cscale(t[m - 1], w.x));
-      im = cadd(im, cscale(d[m - 1], -w.y));
+      re = cfma(t[m - 1], w.x, re);
+      im = m == 1 ? cscale(d[0], -w.y) : cfma(d[m - 1], -w.y, im);
     }
-    const C r = rot<INV>(im);
-    out[q] = cadd(re, r);
-    out[R - q] = csub(re, r);
+    out[q] = cadd_rot<INV>(re, im);
+    out[R - q] = csub_rot<INV>(re, im);
   }
 #pragma unroll
   for (int q = 0; q < R; ++q) v[q] = out[q];
@@ -140,13 +89,13 @@ __device__ __forceinline__ void dft(cplx<T>* v, const cplx<T>* tw, int n) {
     v[0] = cadd(t, v[1]);
     v[1] = csub(t, v[1]);
   } else if constexpr (R == 3) {
-    dft3<T, INV>(v);
+    radix::r3<T, INV>(v);
   } else if constexpr (R == 4) {
-    dft4<INV>(v[0], v[1], v[2], v[3]);
+    radix::r4<INV>(v[0], v[1], v[2], v[3]);
   } else if constexpr (R == 5) {
     dft5<T, INV>(v);
   } else if constexpr (R == 8) {
-    dft8<T, INV>(v);
+    radix::r8<T, INV>(v);
   } else {
     dft_odd<T, INV, R>(v, tw, n);
   }

@@ -21,7 +21,7 @@
 // The adjoint runs the transposes of the same steps.
 // Measured (B200; before: four backward transforms and one forward of the plan
 // around pointwise kernels): physical field to physical field over one RK4
-// step, 192^3 FP32 4172 -> 1666 us; step and gradient, 96^3 FP64 4748 -> 1396 us.
+// step, 192^3 FP32 4172 -> 1615 us; step and gradient, 96^3 FP64 4777 -> 1268 us.
 //
 // Each kernel is two passes of register codelets around one exchange, a kernel
 // per length (as in fft_flex.cuh).  Inverse transforms take the forward
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__((LineShape<T, R1, R2>::NT), (LineShape<T, R1, 
 // Every spectrum element is read once, scaled, and put to both positions of its
 // line that it makes; codelets that loaded their positions themselves read
 // each element twice with index and sign choices per position (192^3 FP32: 221
-// us a launch, 163 us this way).
+// us a launch, 154 us this way).
 template <typename T>
 struct ZArgs {
   Grid g;
