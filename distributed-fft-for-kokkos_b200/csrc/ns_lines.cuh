@@ -21,7 +21,7 @@
 // The adjoint runs the transposes of the same steps.
 // Measured (B200; before: four backward transforms and one forward of the plan
 // around pointwise kernels): physical field to physical field over one RK4
-// step, 192^3 FP32 4172 -> 1615 us; step and gradient, 96^3 FP64 4777 -> 1268 us.
+// step, 192^3 FP32 4172 -> 1579 us; step and gradient, 96^3 FP64 4777 -> 1268 us.
 //
 // Each kernel is two passes of register codelets around one exchange, a kernel
 // per length (as in fft_flex.cuh).  Inverse transforms take the forward
@@ -193,7 +193,8 @@ __global__ void __launch_bounds__((LineShape<T, R1, R2>::NT), (LineShape<T, R1, 
 // Every spectrum element is read once, scaled, and put to both positions of its
 // line that it makes; codelets that loaded their positions themselves read
 // each element twice with index and sign choices per position (192^3 FP32: 221
-// us a launch, 154 us this way).
+// us a launch, 154 us this way, 148 with four
+// elements of a thread in flight).
 template <typename T>
 struct ZArgs {
   Grid g;
@@ -247,29 +248,44 @@ __global__ void __launch_bounds__((ZShape<T, R1, R2, ADJ>::NT), (ZShape<T, R1, R
   // line = pair * NB + field * 3 + component, field 0 A, 1 B, 2 C, 3 D = i k_z A,
   // 4 lambda
   constexpr int NI = ADJ ? 12 : 9;  // lines read: A, B, C (and lambda)
-  for (int it = threadIdx.x; it < npair * NI * kz; it += NT) {
-    int ln, m;
-    split_kz(a.g, it, &ln, &m);
-    const int pr = ln / NI, l = ln % NI;
-    const int64_t pt = 2 * static_cast<int64_t>(pair0 + pr);
-    const bool two = pt + 1 < a.points;
-    const C* x0 = (ADJ && l >= 9 ? a.lambda + static_cast<int64_t>(l - 9) * a.points * kz
-                                 : a.f + static_cast<int64_t>(l) * a.points * kz) + pt * kz + m;
-    const T sc = ADJ && l >= 9 ? T((m == 0 ? 1.0 : 0.5) * a.lscale) : T(a.back);
-    const C c0 = cscale(x0[0], sc), c1 = two ? cscale(x0[kz], sc) : zero;
-    auto put = [&](int line, C p, C q) {
-      C* o = s1 + (pr * NB + line) * P;
-      if (m == 0) {  // the imaginary part of the zero mode dropped
-        o[0] = mk<T>(p.x, q.x);
-      } else {
-        o[m] = mk<T>(p.x - q.y, p.y + q.x);
-        o[N - m] = mk<T>(p.x + q.y, q.x - p.y);
+  constexpr int U = 4;              // items a thread has in flight
+  const int items = npair * NI * kz;
+  for (int it0 = threadIdx.x; it0 < items; it0 += U * NT) {
+    C c0[U], c1[U];
+    int line[U], mode[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int it = min(it0 + u * NT, items - 1);  // (past the end: a load of the last item, not put)
+      int ln;
+      split_kz(a.g, it, &ln, &mode[u]);
+      const int pr = ln / NI, l = ln % NI;
+      const int64_t pt = 2 * static_cast<int64_t>(pair0 + pr);
+      const C* x0 = (ADJ && l >= 9 ? a.lambda + static_cast<int64_t>(l - 9) * a.points * kz
+                                   : a.f + static_cast<int64_t>(l) * a.points * kz) + pt * kz + mode[u];
+      line[u] = pr * NB + l;
+      c0[u] = x0[0];
+      c1[u] = pt + 1 < a.points ? x0[kz] : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (it0 + u * NT >= items) break;
+      const int m = mode[u], l = line[u] % NB;
+      const T sc = ADJ && l >= 9 ? T((m == 0 ? 1.0 : 0.5) * a.lscale) : T(a.back);
+      auto put = [&](int ln, C p, C q) {
+        C* o = s1 + ln * P;
+        if (m == 0) {  // the imaginary part of the zero mode dropped
+          o[0] = mk<T>(p.x, q.x);
+        } else {
+          o[m] = mk<T>(p.x - q.y, p.y + q.x);
+          o[N - m] = mk<T>(p.x + q.y, q.x - p.y);
+        }
+      };
+      const C p = cscale(c0[u], sc), q = cscale(c1[u], sc);
+      put(ADJ && l >= 9 ? line[u] + 3 : line[u], p, q);
+      if (l < 3) {
+        const T k = T(m * a.g.kscale);
+        put(line[u] + 9, ik<T>(k, p), ik<T>(k, q));
       }
-    };
-    put(ADJ && l >= 9 ? l + 3 : l, c0, c1);
-    if (l < 3) {
-      const T k = T(m * a.g.kscale);
-      put(9 + l, ik<T>(k, c0), ik<T>(k, c1));
     }
   }
   __syncthreads();

@@ -88,9 +88,9 @@ class NavierStokes:
 
 def step_graph(states, uks, batched=True):
     """A library-owned CUDA graph of one RK4 step of every field (states[i]
-    advances uks[i]); ``batched``: each transform of all fields batched into
-    one launch per stage, else each field's step on one of up to four
-    concurrent branches.  ``launch(stream)`` advances all fields by one step."""
+    advances uks[i]): each field's step on one of up to four concurrent
+    branches, or, ``batched`` and no field on kept modes, each transform of all
+    fields batched into one launch per stage.  ``launch(stream)`` advances all fields by one step."""
     n = len(states)
     if len(uks) != n or n == 0:
         raise ValueError("one spectral buffer per state")

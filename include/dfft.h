@@ -312,9 +312,11 @@ dfft_status dfft_ns_step(dfft_ns* ns, void* uk, void* stream);
 dfft_status dfft_ns_energy(dfft_ns* ns, const void* uk, double* energy, void* stream);
 /* One RK4 time step of `count` fields (distinct states, uks[i] the spectral
  * buffer of states[i]) captured once into a library-owned CUDA graph.
- *   batched = 1: per RK stage the pointwise phases per field and every
- *     transform of all fields through one batched execution (one launch per
- *     stage of the transform; the states' plans must be distinct);
+ *   batched = 1: where no state's right-hand side runs on kept modes, per RK
+ *     stage the pointwise phases per field and every transform of all fields
+ *     through one batched execution (one launch per stage of the transform);
+ *     else each field's step on one of up to four concurrent graph branches
+ *     (the states' plans must be distinct);
  *   batched = 0: each field's step on one of up to four concurrent graph
  *     branches with its plan's tuned kernels (fields sharing a plan on one
  *     branch).
