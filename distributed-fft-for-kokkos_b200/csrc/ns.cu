@@ -509,30 +509,6 @@ __global__ void ns_scatter_kernel(const DevLayout L, const cplx<T>* a, cplx<T>* 
   }
 }
 
-// mu = P c on kept modes
-template <typename T>
-__global__ void ns_kept_project_kernel(const cplx<T>* c, cplx<T>* mu, NsGeom g, NsKept k) {
-  const int64_t total = static_cast<int64_t>(k.kx) * k.ky * k.kz;
-  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int ix, iy, iz;
-    decode_point(t, k.kz, k.ky, &ix, &iy, &iz);
-    const double kx = (ix <= g.cx ? ix : ix - k.kx) * g.kscale, ky = (iy <= g.cy ? iy : iy - k.ky) * g.kscale,
-                 kz = iz * g.kscale;
-    const double inv_ksq = t == 0 ? 0.0 : 1.0 / (kx * kx + ky * ky + kz * kz);
-    const T ikk = T(inv_ksq);
-    const T kk[3] = {T(kx), T(ky), T(kz)};
-    cplx<T> r[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) r[d] = c[d * total + t];
-    const cplx<T> div = mk<T>((kk[0] * r[0].x + kk[1] * r[1].x + kk[2] * r[2].x) * ikk,
-                              (kk[0] * r[0].y + kk[1] * r[1].y + kk[2] * r[2].y) * ikk);
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      mu[d * total + t] = mk<T>(r[d].x - kk[d] * div.x, r[d].y - kk[d] * div.y);
-  }
-}
-
 // y = a + s x over whole buffers (n complex elements)
 template <typename T>
 __global__ void ns_axpy_kernel(const cplx<T>* a, const cplx<T>* x, cplx<T>* y, double s, int64_t n) {
@@ -575,11 +551,11 @@ struct NsState {
   void* ladv = nullptr;
   // the right-hand side on kept modes (null: the plan's transforms), its
   // spectra: y0, the stage state, k1, k2, k3; of the adjoint: 4 stage states
-  // (the first is y0), mu, lambda, the cotangents of y0 and k, the VJP
+  // (the first is y0), mu, lambda, the cotangent of y0, the VJP
   std::unique_ptr<NsLines> lines;
   dev::NsKept kept{};
   void* kept_rk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  void* kept_adj[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  void* kept_adj[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   ~NsState() {
     for (auto p : kept_rk) cudaFree(p);
     for (auto p : kept_adj) cudaFree(p);
@@ -1155,34 +1131,27 @@ static bool ns_kept_adjoint(NsState* s) {
   return true;
 }
 
-template <typename T>
-static void ns_kept_vjp(NsState* s, const void* y, const void* c, void* out, cudaStream_t st) {
-  using namespace dev;
-  using C = cplx<T>;
-  void* mu = s->kept_adj[3];
-  const int64_t n = static_cast<int64_t>(s->kept.kx) * s->kept.ky * s->kept.kz;
-  ns_kept_project_kernel<T><<<grid_of(n), 256, 0, st>>>(static_cast<const C*>(c), static_cast<C*>(mu), s->g, s->kept);
-  ck(cudaGetLastError(), "ns vjp projection");
-  s->lines->vjp(y, mu, out, s->nu, st);
-}
-
-template <typename T>
 static void ns_kept_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cudaStream_t st) {
-  void *y = s->kept_rk[0], *c = s->kept_adj[4], *out = s->kept_adj[7];
+  void *y = s->kept_rk[0], *c = s->kept_adj[4], *out = s->kept_adj[6];
   ns_gather(s, uk, y, st);
   ns_gather(s, lam, c, st);
-  ns_kept_vjp<T>(s, y, c, out, st);
+  NsLines::Vjp v;
+  v.y = y;
+  v.mu = s->kept_adj[3];
+  v.nu = s->nu;
+  v.out = out;
+  s->lines->project(c, v.mu, 1.0, st);
+  s->lines->vjp(v, st);
   ns_scatter(s, out, grad, st);
 }
 
 // As ns_step_adjoint_t, on kept modes: the stage states a_i = a_1 + up h f(a_{i-1})
-// come straight out of the right-hand side's last kernel.
-template <typename T>
+// come straight out of the right-hand side's last kernel, the cotangents out
+// of the VJP's.
 static void ns_kept_step_adjoint(NsState* s, const void* uk, void* lam, cudaStream_t st) {
   const double h = s->dt;
-  const std::size_t n = s->lines->elements();
   void* a[4] = {s->kept_rk[0], s->kept_adj[0], s->kept_adj[1], s->kept_adj[2]};
-  void *l = s->kept_adj[4], *ly0 = s->kept_adj[5], *lk = s->kept_adj[6], *g = s->kept_adj[7];
+  void *l = s->kept_adj[4], *ly0 = s->kept_adj[5];
   ns_gather(s, uk, a[0], st);
   ns_gather(s, lam, l, st);
   const double up[3] = {0.5, 0.5, 1.0};  // a2 = a1 + k1 / 2, a3 = a1 + k2 / 2, a4 = a1 + k3
@@ -1197,25 +1166,28 @@ static void ns_kept_step_adjoint(NsState* s, const void* uk, void* lam, cudaStre
     s->lines->rhs(w, st);
   }
   const double direct[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};  // d S / d k_i
-  launch_axpy<T>(l, l, lk, direct[3] - 1.0, n, st);
+  NsLines::Vjp v;
+  v.mu = s->kept_adj[3];
+  v.nu = s->nu;
+  v.l = l;
+  v.ly0 = ly0;
+  v.h = h;
+  s->lines->project(l, v.mu, direct[3], st);  // the cotangent of k_4
   for (int i = 3; i >= 0; --i) {
-    // g = f'(a_i)^T lk
-    ns_kept_vjp<T>(s, a[i], lk, g, st);
-    launch_axpy<T>(i == 3 ? l : ly0, g, ly0, h, n, st);
-    if (i > 0) {
-      launch_axpy<T>(l, l, lk, direct[i - 1] - 1.0, n, st);
-      launch_axpy<T>(lk, g, lk, h * up[i - 1], n, st);
-    }
+    // g = f'(a_i)^T lk; the cotangent of k_i (1-based) its direct weight in S
+    // plus up[i - 1] times this stage's h g
+    v.y = a[i];
+    v.first = i == 3;
+    v.direct = i > 0 ? direct[i - 1] : 0.0;
+    v.up = i > 0 ? up[i - 1] : 0.0;
+    s->lines->vjp(v, st);
   }
   ns_scatter(s, ly0, lam, st);
 }
 
 void ns_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cudaStream_t st) {
   if (ns_kept_adjoint(s)) {
-    if (s->dbl)
-      ns_kept_rhs_adjoint<double>(s, uk, lam, grad, st);
-    else
-      ns_kept_rhs_adjoint<float>(s, uk, lam, grad, st);
+    ns_kept_rhs_adjoint(s, uk, lam, grad, st);
     return;
   }
   if (s->dbl)
@@ -1226,10 +1198,7 @@ void ns_rhs_adjoint(NsState* s, const void* uk, const void* lam, void* grad, cud
 
 void ns_step_adjoint(NsState* s, const void* uk, void* lam, cudaStream_t st) {
   if (ns_kept_adjoint(s)) {
-    if (s->dbl)
-      ns_kept_step_adjoint<double>(s, uk, lam, st);
-    else
-      ns_kept_step_adjoint<float>(s, uk, lam, st);
+    ns_kept_step_adjoint(s, uk, lam, st);
     return;
   }
   if (s->dbl)

@@ -21,7 +21,7 @@
 // The adjoint runs the transposes of the same steps.
 // Measured (B200; before: four backward transforms and one forward of the plan
 // around pointwise kernels): physical field to physical field over one RK4
-// step, 192^3 FP32 4172 -> 1579 us; step and gradient, 96^3 FP64 4777 -> 1268 us.
+// step, 192^3 FP32 4172 -> 1579 us; step and gradient, 96^3 FP64 4771 -> 1216 us.
 //
 // Each kernel is two passes of register codelets around one exchange, a kernel
 // per length (as in fft_flex.cuh).  Inverse transforms take the forward

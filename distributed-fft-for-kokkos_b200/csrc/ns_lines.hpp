@@ -37,8 +37,22 @@ class NsLines {
     int step = 4;
   };
   virtual void rhs(const Update& w, cudaStream_t st) = 0;
-  // out = (d f / d u at y)^T c with mu = P c given
-  virtual void vjp(const void* y, const void* mu, void* out, double nu, cudaStream_t st) = 0;
+  // g = (d f / d u at y)^T c with mu = P c given, and what becomes of it
+  struct Vjp {
+    const void* y = nullptr;
+    void* mu = nullptr;
+    double nu = 0.0;
+    void* out = nullptr;  // out = g; or, null, one stage of an RK4 step backwards:
+    // ly0 <- (first: l, else ly0) + h g, and, if direct != 0, the next stage's
+    // mu <- P(direct l + h up g)
+    const void* l = nullptr;
+    void* ly0 = nullptr;
+    double h = 0.0, direct = 0.0, up = 0.0;
+    bool first = false;
+  };
+  virtual void vjp(const Vjp& w, cudaStream_t st) = 0;
+  // mu = P(s c)
+  virtual void project(const void* c, void* mu, double s, cudaStream_t st) = 0;
 };
 
 }  // namespace dfft
