@@ -14,7 +14,7 @@
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
 // kernels): 300 x 250 x 360 complex64 3818 -> 544 us, 200 x 180 x 252 R2C / C2R
 // double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 155 us, 256^3
-// complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1158 us.  On 2^k and
+// complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1131 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
 //
@@ -45,15 +45,18 @@ namespace flex {
 using codelet::Dft;
 
 // Resident threads per SM the registers are sized for: what the R1 values of a
-// thread, its addresses and the codelet's temporaries take without spilling
-// (more for C2R lines, which load both half spectra, and for the chirp-z form).
+// thread, its addresses and the codelet's temporaries take with at most a few
+// spills (more for the chirp-z form, `more`).  C2R lines, which load both half
+// spectra, take a few more registers when left alone, and lose a CTA per SM by
+// it (384^3 double: 221 us a launch at two CTAs of 210 registers, 186 at four).
 template <typename T>
-constexpr int resident_threads(int r, bool more) {
+constexpr int resident_threads(int r, bool more, bool afast = false) {
   if (sizeof(T) == 4)
     return more ? (r <= 12 ? 896 : r <= 16 ? 768 : r <= 21 ? 576 : 512)
                 : (r <= 8 ? 1280 : r <= 12 ? 1024 : r <= 16 ? 896 : r <= 21 ? 640 : r <= 25 ? 576 : 512);
-  return more ? (r <= 8 ? 768 : r <= 10 ? 640 : r <= 12 ? 512 : r <= 16 ? 512 : r <= 21 ? 384 : r <= 25 ? 320 : 256)
-              : (r <= 8 ? 896 : r <= 10 ? 768 : r <= 12 ? 640 : r <= 16 ? 512 : r <= 21 ? 448 : r <= 25 ? 384 : 256);
+  return more ? (r <= 8 ? 768 : r <= 10 ? 640 : r <= 16 ? 512 : r <= 21 ? 384 : r <= 25 ? 320 : 256)
+              : (r <= 8 ? 896 : r <= 10 ? 768 : r <= 12 ? 640 : r <= 16 ? 512 : r <= 21 ? 448
+                 : r <= 24 && afast ? 512 : r <= 25 ? 384 : 256);
 }
 
 // Lines per tile: about 128 threads.  b-fast rows of 128 bytes; of 64 bytes for
@@ -78,7 +81,7 @@ struct Shape {
   static constexpr int p1 = R2 * odd1, p2 = CHIRP ? R1 * odd2 : 0, pn = m | 1;
   static constexpr int P = AFAST ? (p1 > p2 ? (p1 > pn ? p1 : pn) : (p2 > pn ? p2 : pn)) : m;
   static constexpr size_t smem = sizeof(cplx<T>) * B * P;
-  static constexpr int fit = resident_threads<T>(R1, CHIRP || KIND == kC2R) / NT;
+  static constexpr int fit = resident_threads<T>(R1, CHIRP, AFAST) / NT;
   static constexpr int blocks = fit > 0 ? fit : 1;
 };
 
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
     } else if constexpr (KIND == kC2R) {
       // Z from the half spectra directly, every mode loaded for both positions
       // it makes: through shared memory as in the chirp-z form, with its
-      // barriers, 384^3 double took 273 us instead of 221 (131 x 105 x 157
+      // barriers, 384^3 double took 273 us where this form took 221 (131 x 105 x 157
       // chirp-z lines, where the loads' index choices weigh more, 36 instead of
       // 46)
       const bool two = 2 * line2 + 1 < nb;
