@@ -444,7 +444,7 @@ def main():
     # per-field transforms on concurrent graph branches (dfft_graph_create)
     bgraph = dfft.Graph(items)
     ms_branch32 = timed_launch(lambda: bgraph.launch(stream.cuda_stream))
-    # one persistent launch per stage of all 16 fields (dfft_batch_execute),
+    # one launch per stage and line length of all 16 fields (dfft_batch_execute),
     # forward + backward captured in one CUDA graph
     fb = dfft.Batch([f[0] for f in batch["float32"]])
     xs, ys, zs = ([f[k] for f in batch["float32"]] for k in (1, 2, 3))
@@ -488,8 +488,7 @@ def main():
             fl.append((pl, st, uk))
         ns_fields[prec] = fl
     torch.cuda.synchronize()
-    # one RK4 step of all 16 fields in a library-owned CUDA graph: every
-    # transform of all fields batched into one launch per stage
+    # one RK4 step of all 16 fields in a library-owned CUDA graph
     # (dfft_ns_graph_create)
     ns_steps = max(3, args.steps // 20)
     ms_ns = {}

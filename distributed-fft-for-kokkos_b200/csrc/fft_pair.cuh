@@ -198,12 +198,10 @@ __device__ __forceinline__ void store_pair(const StageArgs& A, float2* out, int6
 // One tile (tile tb along b, coordinates co0 / co1) of a two-line C2C stage:
 // PB line pairs, N/8 threads per pair, `smem_raw` holding N complex64
 // twiddles and PB * LP 16-byte line elements (pair_tile_smem).  Called by
-// fft_pair_kernel (one tile per CTA) and by the batched stage kernels, whose
-// CTAs walk tiles of many fields (stage_tw = false: the twiddles of this N
-// are already staged).  Separable sides only.
+// fft_pair_kernel and by the batched stage kernels, one tile per CTA.
+// Separable sides only.
 template <bool INV, int N, int PB, bool AFAST, bool COMP = false, bool ATAB = false>
-__device__ __forceinline__ void pair_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw,
-                                          bool stage_tw = true) {
+__device__ __forceinline__ void pair_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw) {
   using C = float2;
   constexpr int V = 8;
   static_assert(Vals<N>::value == V, "two-line kernel: lines of 2^k points");
@@ -227,7 +225,7 @@ __device__ __forceinline__ void pair_tile(const StageArgs& A, int tb, int co0, i
   const int l0 = AFAST ? lp : 2 * lp, l1 = AFAST ? lp + PB : 2 * lp + 1;
   const bool act0 = l0 < nb, act1 = l1 < nb;
 
-  if (stage_tw) {
+  {
     const C* gtw = reinterpret_cast<const C*>(A.tw);
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
   }

@@ -1,7 +1,7 @@
 // Tile bodies of the register-resident stages (one line per thread group):
 // fast_tile (C2C, lines of 2^k or 3 * 2^k points) and real_tile (R2C first /
 // C2R last stage, two real lines per register line).  fft_fast.cu launches
-// one tile per CTA; fft_batch.cu's persistent CTAs walk tiles of many fields.
+// the tiles of one field, fft_batch.cu those of many.
 #pragma once
 
 #include "fft_radix.cuh"
@@ -12,13 +12,10 @@ namespace radix {
 
 // One tile (tile tb along b, coordinates co0 / co1 along o0 / o1) of a C2C
 // stage, run by N/V*B threads with `smem_raw` of (N + B*LP) complex elements.
-// Called by fft_fast_kernel (one tile per CTA) and by the batched stage
-// kernels (fft_batch.cu), whose CTAs walk tiles of several fields.
+// Called by fft_fast_kernel and by the batched stage kernels (fft_batch.cu),
+// one tile per CTA.
 template <typename T, bool INV, int N, int B, bool AFAST, bool AFF>
-// stage_tw = false: the twiddles of this N are already in smem_raw (the
-// previous tile of the CTA had the same line length)
-__device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw,
-                                          bool stage_tw = true) {
+__device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw) {
   using C = cplx<T>;
   constexpr int V = Vals<N>::value;
   constexpr int TT = N / V;                  // threads per line
@@ -45,8 +42,7 @@ __device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, i
 
   {
     const C* gtw = reinterpret_cast<const C*>(A.tw);
-    if (stage_tw)
-      for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
+    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
   }
 
   // offsets shared by the whole tile (separable tables)
@@ -223,8 +219,7 @@ __device__ __forceinline__ void fast_tile(const StageArgs& A, int tb, int co0, i
 //        dropped), inverse FFT, x0 = Re z and x1 = Im z are written.
 // The interior modes (all but DC and Nyquist) carry the factor A.weight.
 template <typename T, bool C2R, int N, int B, bool AFF>
-__device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw,
-                                          bool stage_tw = true) {
+__device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, int co1, unsigned char* smem_raw) {
   using C = cplx<T>;
   constexpr int V = Vals<N>::value;
   constexpr int TT = N / V;
@@ -247,8 +242,7 @@ __device__ __forceinline__ void real_tile(const StageArgs& A, int tb, int co0, i
 
   {
     const C* gtw = reinterpret_cast<const C*>(A.tw);
-    if (stage_tw)
-      for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
+    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
   }
   // row bases (offset of position 0 of each real / complex line); lines are
   // contiguous along a on both sides
