@@ -116,7 +116,9 @@ inline cudaError_t launch_kernel_early(bool early, void (*kernel)(P...), dim3 gr
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch's check
+  return e;
 }
 
 // a stage's early start: by the bytes of the array it reads (complex elements)
