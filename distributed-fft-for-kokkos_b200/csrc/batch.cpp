@@ -28,9 +28,9 @@ using GroupKey = std::tuple<int, bool, bool, int, bool>;
 
 // complex64 C2C stages the one-tile launches would run two lines per thread
 // (separable sides, pair-aligned: op.single_B is set) take the batched
-// two-line tiles
+// two-line tiles (which address positions by stride only)
 bool pair_batchable(const Op& op, bool dbl) {
-  return !dbl && op.kind == dev::kC2C && op.single_B != 0 && dev::batch_pair_lines(op.sa.n, op.sa.load_afast != 0) > 0;
+  return !dbl && op.kind == dev::kC2C && op.single_B != 0 && !op.sa.src_atab && !op.sa.dst_atab && dev::batch_pair_lines(op.sa.n, op.sa.load_afast != 0) > 0;
 }
 
 void ck(cudaError_t e) {

@@ -4,6 +4,7 @@
 // KOKKOSFFT_THROW_IF; nothing may unwind across a C ABI).
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -423,6 +424,44 @@ dfft_status dfft_debug_export_buffers(const dfft_plan* plan, int32_t direction, 
     if (block < 0) dfft::fail(dfft::kErrInvalidArgument, "block index out of range");
     impl_of(plan).export_buffers(direction == DFFT_FORWARD, static_cast<std::size_t>(block), which, host_dst,
                                  capacity_bytes);
+  });
+}
+
+dfft_status dfft_debug_get_stage(const dfft_plan* plan, int32_t program, int64_t step, dfft_stage_info* info) {
+  return guarded([&] {
+    if (!info) dfft::fail(dfft::kErrInvalidArgument, "null output");
+    if (program < 0 || program > 3) dfft::fail(dfft::kErrInvalidArgument, "program must be 0 to 3");
+    const dfft::Plan& given = impl_of(plan);
+    std::unique_ptr<dfft::Plan> host;  // the programs of a host-only plan, built for this call
+    if (!given.on_device()) host = std::make_unique<dfft::Plan>(given.desc(), false, true);
+    const dfft::Plan& p = host ? *host : given;
+    const auto& ops = program < 2 ? p.program(program == 0) : p.adjoint_program(program == 2);
+    if (step < 0 || static_cast<std::size_t>(step) >= ops.size())
+      dfft::fail(dfft::kErrInvalidArgument, "step index out of range");
+    const dfft::Op& op = ops[static_cast<std::size_t>(step)];
+    const dfft::dev::StageArgs& A = op.sa;
+    *info = dfft_stage_info{};
+    if (op.type != dfft::Op::Stage || op.kind > dfft::dev::kC2R) {
+      info->kernel = DFFT_KERNEL_OTHER;
+      return;
+    }
+    info->kernel = A.pairs == 4   ? (op.chirp ? DFFT_KERNEL_TWO_PASS_CHIRP : DFFT_KERNEL_TWO_PASS)
+                   : A.pairs == 3 ? DFFT_KERNEL_PAIR_TMA
+                   : A.pairs == 2 ? DFFT_KERNEL_PAIR_STREAM
+                   : A.pairs == 1 ? DFFT_KERNEL_PAIR
+                   : op.fast      ? DFFT_KERNEL_REGISTER
+                                  : DFFT_KERNEL_TABLE;
+    info->n = A.n;
+    info->two_pass = op.flex ? 1 : 0;
+    info->lines = A.B;
+    info->general[0] = A.src_line_affine;
+    info->general[1] = A.dst_line_affine;
+    info->axis_table[0] = A.src_atab;
+    info->axis_table[1] = A.dst_atab;
+    info->base[0] = A.src_abase;
+    info->base[1] = A.dst_abase;
+    info->stride[0] = A.src_astride;
+    info->stride[1] = A.dst_astride;
   });
 }
 

@@ -407,7 +407,8 @@ int pair_tma_line_options(int n, int* opts) {
 
 cudaError_t launch_fft_pair_tma(const StageArgs& A, const void* map, const TmaCoords& T, bool inverse,
                                 cudaStream_t st) {
-  if (!A.err) return cudaErrorInvalidValue;
+  // (the kernel addresses positions by stride only)
+  if (!A.err || A.src_atab || A.dst_atab) return cudaErrorInvalidValue;
   switch (A.n) {
 #define DFFT_TMA(N_) \
   case N_: return inverse ? launch_tma_n<N_, true>(A, map, T, st) : launch_tma_n<N_, false>(A, map, T, st);

@@ -156,7 +156,7 @@ void host_dft(std::vector<long double>& re, std::vector<long double>& im) {
 // ---------------------------------------------------------------------------
 // Construction
 // ---------------------------------------------------------------------------
-Plan::Plan(const PlanDesc& d, bool on_device) : d_(d), on_device_(on_device) {
+Plan::Plan(const PlanDesc& d, bool on_device, bool programs) : d_(d), on_device_(on_device) {
   analyze();
   if (is_rank_plan()) {
     if (static_cast<std::size_t>(d_.rank) >= nprocs())
@@ -165,25 +165,24 @@ Plan::Plan(const PlanDesc& d, bool on_device) : d_(d), on_device_(on_device) {
     rank_exchanges(true);
     rank_exchanges(false);
   }
-  if (!on_device_) return;
+  if (!on_device_ && !programs) return;
   try {
     if (is_rank_plan()) {
       build_rank(true);
       build_rank(false);
-      allocate_device();
-      autotune();
-      return;
+    } else {
+      build_fused(true);
+      build_fused(false);
+      build_adjoint(true);
+      build_adjoint(false);
+      if (d_.exec_mode == 1 || d_.exec_mode == 2) {
+        prog_[0].clear();
+        prog_[1].clear();
+        build_literal(true);
+        build_literal(false);
+      }
     }
-    build_fused(true);
-    build_fused(false);
-    build_adjoint(true);
-    build_adjoint(false);
-    if (d_.exec_mode == 1 || d_.exec_mode == 2) {
-      prog_[0].clear();
-      prog_[1].clear();
-      build_literal(true);
-      build_literal(false);
-    }
+    if (!on_device_) return;
     allocate_device();
     autotune();
   } catch (...) {
@@ -346,6 +345,7 @@ std::vector<std::size_t> Plan::fft_axis_order() const {
 }
 
 const void* Plan::twiddle(std::size_t n) {
+  if (!on_device_) return nullptr;
   auto key = std::make_pair(n, d_.dbl);
   auto it = twiddles_.find(key);
   if (it != twiddles_.end()) return it->second;
@@ -417,12 +417,50 @@ void Plan::select_flex(Op& op) const {
   op.tiles = static_cast<unsigned>(static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1);
 }
 
+// How the line kernels address the lines along axis `a` of one side of a
+// stage: base + position * stride from the separable offset tables (affine = 0;
+// unit stride when the lines are read along a), the same from the general ones
+// (affine = 1: no rank block splits a), or position by position from the axis
+// table (atab = 1; `tables`: any separable side, else only exchange buffers
+// split into bins along a).  The register kernels and the two-pass kernel of a
+// stage share what this returns: a kernel that addresses lines by stride and
+// one that reads the table must not see each other's fields.  False: neither.
+bool Plan::line_side(int l, std::size_t a, bool afast, bool tables, LineSide* s) const {
+  const Layout& L = layouts_[l];
+  const LayoutTables& T = tables_[l];
+  const std::size_t len = L.gext[a];
+  *s = LineSide{};
+  if (T.mode != 0) {
+    s->affine = 1;
+    return L.topo[a] == 1 && (!afast || layout_fast_axis(L) == a);
+  }
+  const std::int64_t* off = T.data.data() + T.off[a];
+  const std::int64_t st = len > 1 ? off[1] - off[0] : 1;
+  bool aff = !afast || st == 1;
+  for (std::size_t c = 1; aff && c < len; ++c)
+    if (off[c] != off[0] + static_cast<std::int64_t>(c) * st) aff = false;
+  // the kernels take 32-bit offsets along a line
+  if (aff && static_cast<std::int64_t>(len - 1) * (st < 0 ? -st : st) >= (std::int64_t(1) << 31)) aff = false;
+  if (aff) {
+    s->base = off[0];
+    s->stride = st;
+    return true;
+  }
+  if ((tables || (!L.pad.empty() && L.topo[a] > 1)) && (!afast || layout_fast_axis(L) == a)) {
+    s->atab = 1;  // the table carries the whole offset along a
+    return true;
+  }
+  return false;
+}
+
 // The two-pass kernel for a stage whose geometry (axes, extents, row
 // orientation) is set: lengths that have a kernel (fft_flex_lengths.h), or
 // whose chirp-z convolution does; rows of one orientation on both sides; every
 // side addressable by line: separable tables (R2C / C2R: lines in one piece),
-// or general ones whose rank blocks do not split a.  Fills op.fx and the line
-// addressing; false (op untouched) if the kernel does not take the stage.
+// or general ones whose rank blocks do not split a.  A stage that has a
+// register kernel (op.fast) keeps the addressing it has: the kernel takes that
+// or not the stage.  Else this fills it.  False (op untouched) if the kernel
+// does not take the stage.
 bool Plan::add_flex(Op& op) {
   dev::StageArgs& A = op.sa;
   const std::size_t a = static_cast<std::size_t>(A.a);
@@ -432,37 +470,18 @@ bool Plan::add_flex(Op& op) {
     return false;
   const int nh = A.n / 2 + 1;
   if (A.na_in != (op.kind == dev::kC2R ? nh : A.n) || A.na_out != (op.kind == dev::kR2C ? nh : A.n)) return false;
-  struct Side {
-    int affine = 0, atab = 0;
-    std::int64_t base = 0, stride = 1;
-  } side[2];
+  LineSide side[2] = {{A.src_line_affine, A.src_atab, A.src_abase, A.src_astride},
+                      {A.dst_line_affine, A.dst_atab, A.dst_abase, A.dst_astride}};
   for (int k = 0; k < 2; ++k) {
     const int l = k == 0 ? op.src_layout : op.dst_layout;
-    const LayoutTables& T = tables_[l];
-    const std::size_t len = layouts_[l].gext[a];
-    Side& s = side[k];
-    // the kernels take the offsets along a line (32 bits), unit stride when a-fast
-    if (afast && layout_fast_axis(layouts_[l]) != a) return false;
-    if (T.mode != 0) {
-      if (layouts_[l].topo[a] != 1) return false;
-      s.affine = 1;
-      for (const RankBlock& rb : layout_blocks(layouts_[l]))
-        if (static_cast<std::int64_t>(len) * static_cast<std::int64_t>(rb.stride[a]) >= (std::int64_t(1) << 31))
-          return false;
-      continue;
-    }
-    const std::int64_t* off = T.data.data() + T.off[a];
-    s.stride = len > 1 ? off[1] - off[0] : 1;
-    s.base = off[0];
-    for (std::size_t c = 1; c < len; ++c)
-      if (off[c] != off[0] + static_cast<std::int64_t>(c) * s.stride) s.atab = 1;
-    if (afast && s.stride != 1) s.atab = 1;
-    if (s.stride < 0 || static_cast<std::int64_t>(len) * s.stride >= (std::int64_t(1) << 31)) s.atab = 1;
-    if (s.atab) {
-      if (real) return false;
-      s.base = 0;  // the table carries the whole offset along a
-      s.stride = 1;
-    }
+    if (!op.fast && !line_side(l, a, afast, !real, &side[k])) return false;
+    if (real && side[k].atab) return false;
+    if (!side[k].affine) continue;
+    // general tables: the kernel takes 32-bit offsets along a line
+    for (const RankBlock& rb : layout_blocks(layouts_[l]))
+      if (static_cast<std::int64_t>(layouts_[l].gext[a] - 1) * static_cast<std::int64_t>(rb.stride[a]) >=
+          (std::int64_t(1) << 31))
+        return false;
   }
   int r1 = 0, r2 = 0;
   const bool chirp = !radix_supported(static_cast<std::size_t>(A.n));
@@ -479,15 +498,19 @@ bool Plan::add_flex(Op& op) {
   if (chirp)
     bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &op.fx.chirp, &op.fx.filter,
                      &op.fx.filter_inverse);
-  A.src_line_affine = side[0].affine;
-  A.src_atab = side[0].atab;
-  A.src_abase = side[0].base;
-  A.src_astride = side[0].stride;
-  A.dst_line_affine = side[1].affine;
-  A.dst_atab = side[1].atab;
-  A.dst_abase = side[1].base;
-  A.dst_astride = side[1].stride;
+  if (!op.fast) set_lines(A, side[0], side[1]);
   return true;
+}
+
+void Plan::set_lines(dev::StageArgs& A, const LineSide& src, const LineSide& dst) {
+  A.src_line_affine = src.affine;
+  A.src_atab = src.atab;
+  A.src_abase = src.base;
+  A.src_astride = src.stride;
+  A.dst_line_affine = dst.affine;
+  A.dst_atab = dst.atab;
+  A.dst_abase = dst.base;
+  A.dst_astride = dst.stride;
 }
 
 // Chirp and filter tables of an n-point chirp-z stage with m-point FFTs, in
@@ -496,6 +519,8 @@ bool Plan::add_flex(Op& op) {
 // for 0 < j < n and 0 elsewhere, the inverse filter the same for the
 // conjugate chirp.  Computed in long double on the host.
 void Plan::bluestein_tables(std::size_t n, std::size_t m, const void** chirp, const void** ffwd, const void** finv) {
+  *chirp = *ffwd = *finv = nullptr;
+  if (!on_device_) return;
   auto key = std::make_pair(n, m);
   auto it = blue_tables_.find(key);
   if (it == blue_tables_.end()) {
@@ -759,51 +784,16 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
   // contiguous run) or general tables whose rank blocks do not split axis a
   // (every line is affine, base + p * stride; lines read along a have unit
   // stride because a is the layout's fast axis).
-  auto side_ok = [&](int l, const Layout& L, std::size_t len, bool afast, int* affine, int* atab,
-                     std::int64_t* abase, std::int64_t* astride) {
-    const LayoutTables& T = tables_[l];
-    *atab = 0;
-    if (T.mode == 0) {
-      // separable: the offsets along a must be affine (unit stride when the
-      // lines are read along a)
-      *affine = 0;
-      const std::int64_t* off = T.data.data() + T.off[a];
-      const std::int64_t st = len > 1 ? off[1] - off[0] : 1;
-      bool aff = !afast || st == 1;
-      for (std::size_t c = 1; aff && c < len; ++c)
-        if (off[c] != off[0] + static_cast<std::int64_t>(c) * st) aff = false;
-      // the kernels take 32-bit offsets along a line
-      if (aff && static_cast<std::int64_t>(len - 1) * (st < 0 ? -st : st) >= (std::int64_t(1) << 31)) aff = false;
-      if (aff) {
-        *abase = off[0];
-        *astride = st;
-        return true;
-      }
-      // an exchange buffer split into bins along a (per-rank programs): the
-      // general-layout kernel variant reads positions from the axis table
-      if (!L.pad.empty() && L.topo[a] > 1 && (!afast || layout_fast_axis(L) == a)) {
-        *atab = 1;
-        *abase = 0;
-        *astride = 1;
-        return true;
-      }
-      return false;
-    }
-    *affine = 1;
-    return L.topo[a] == 1 && (!afast || layout_fast_axis(L) == a);
-  };
   // the register kernels take the coordinates along o0 / o1 from a grid of
   // (tiles, Eo0, Eo1) CTAs
   const bool grid_ok = A.Eo0 <= dev::fast_stage_max_grid_yz() && A.Eo1 <= dev::fast_stage_max_grid_yz();
   const std::size_t Bf = (grid_ok && dev::fast_stage_supported(static_cast<int>(n)))
                              ? static_cast<std::size_t>(dev::fast_stage_lines(d_.dbl, static_cast<int>(n)))
                              : 0;
-  int saff = 0, daff = 0, satab = 0, datab = 0;
-  std::int64_t sab = 0, sas = 0, dab = 0, das = 0;
+  LineSide ss, sd;
   // C2C: lines of n points on both sides, the same row orientation
   if (kind == dev::kC2C && Bf && A.load_afast == A.store_afast && S.gext[a] == n && Dl.gext[a] == n &&
-      side_ok(src_l, S, n, A.load_afast != 0, &saff, &satab, &sab, &sas) &&
-      side_ok(dst_l, Dl, n, A.load_afast != 0, &daff, &datab, &dab, &das)) {
+      line_side(src_l, a, A.load_afast != 0, false, &ss) && line_side(dst_l, a, A.load_afast != 0, false, &sd)) {
     op.fast = true;
     A.B = static_cast<int>(Bf);
     A.tiles_b = static_cast<int>((Dl.gext[b] + Bf - 1) / Bf);
@@ -813,21 +803,13 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
   const std::size_t nr = n, nc = n / 2 + 1;
   const std::size_t ns = kind == dev::kR2C ? nr : nc, ndst = kind == dev::kR2C ? nc : nr;
   if ((kind == dev::kR2C || kind == dev::kC2R) && Bf && A.load_afast && A.store_afast && S.gext[a] == ns &&
-      Dl.gext[a] == ndst && side_ok(src_l, S, ns, true, &saff, &satab, &sab, &sas) &&
-      side_ok(dst_l, Dl, ndst, true, &daff, &datab, &dab, &das)) {
+      Dl.gext[a] == ndst && line_side(src_l, a, true, false, &ss) && line_side(dst_l, a, true, false, &sd)) {
     op.fast = true;
     A.B = static_cast<int>(Bf);
     A.tiles_b = static_cast<int>((Dl.gext[b] + 2 * Bf - 1) / (2 * Bf));
   }
   if (op.fast) {
-    A.src_line_affine = saff;
-    A.dst_line_affine = daff;
-    A.src_atab = satab;
-    A.dst_atab = datab;
-    A.src_abase = sab;
-    A.src_astride = sas;
-    A.dst_abase = dab;
-    A.dst_astride = das;
+    set_lines(A, ss, sd);
     // Two complex64 lines per thread: C2C of 2^k points on separable sides;
     // b-fast tiles move both lines of a pair with one 16-byte access, so
     // every pair must start on an even element on both sides.
@@ -855,9 +837,10 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
     };
     // (axis-table sides: the two-line kernel takes the positions along a from
     // the table; b-fast pairs need every offset even)
-    const bool atab = satab || datab;
-    if (kind == dev::kC2C && !d_.dbl && dev::pair_stage_supported(static_cast<int>(n)) && !saff && !daff &&
-        (A.load_afast || (pair_aligned(src_l, sab, sas, satab) && pair_aligned(dst_l, dab, das, datab)))) {
+    const bool atab = ss.atab || sd.atab;
+    if (kind == dev::kC2C && !d_.dbl && dev::pair_stage_supported(static_cast<int>(n)) && !ss.affine && !sd.affine &&
+        (A.load_afast || (pair_aligned(src_l, ss.base, ss.stride, ss.atab) &&
+                          pair_aligned(dst_l, sd.base, sd.stride, sd.atab)))) {
       int opts[3];
       dev::pair_stage_line_options(static_cast<int>(n), A.load_afast != 0, opts);
       op.single_B = A.B;
@@ -881,8 +864,7 @@ Op Plan::make_stage(int src_l, int dst_l, std::size_t a, int kind, bool inverse,
     const unsigned long long ft = static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1;
     if (ft >= (1ull << 31)) fail(kErrUnsupported, "too many tiles");
     op.tiles = static_cast<unsigned>(ft);
-    // the two-pass kernel as another variant for the tuner (it computes the
-    // same line addressing)
+    // the two-pass kernel as another variant for the tuner
     if (!A.comp) add_flex(op);
   } else if (!is_copy && add_flex(op)) {
     select_flex(op);
@@ -1467,7 +1449,7 @@ void Plan::autotune() {
       std::ostringstream k;
       const bool real = op.kind == dev::kR2C || op.kind == dev::kC2R;  // two real lines per register line
       const bool pair_ok = op.single_B != 0;                            // eligible for two lines per thread
-      const bool tma_ok = op.tma.ok;                                    // eligible for the TMA-fed kernel
+      const bool tma_ok = op.tma.ok && !A.src_atab && !A.dst_atab;      // eligible for the TMA-fed kernel
       k << (op.flex ? "fast+flex:n" : "fast:n") << A.n << (d_.dbl ? "f64" : "f32") << (op.inverse ? "i" : "f") << (A.load_afast ? "a" : "b")
         << (op.kind == dev::kR2C ? "r2c" : op.kind == dev::kC2R ? "c2r" : "") << (pair_ok ? "P" : "")
         << (tma_ok ? "T" : "") << (A.comp ? "C" : "")

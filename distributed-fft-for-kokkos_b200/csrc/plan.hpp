@@ -119,7 +119,8 @@ struct Op {
 
 class Plan {
  public:
-  Plan(const PlanDesc& d, bool on_device);
+  // programs: build the programs of a host-only plan too (dfft_debug_get_stage)
+  Plan(const PlanDesc& d, bool on_device, bool programs = false);
   ~Plan();
   Plan(const Plan&) = delete;
   Plan& operator=(const Plan&) = delete;
@@ -149,6 +150,7 @@ class Plan {
   // Batched execution (batch.cpp): the fused program of a direction, the
   // plan's device buffers by id, one op's launch, and the checks of execute.
   const std::vector<Op>& program(bool forward) const { return prog_[forward ? 0 : 1]; }
+  const std::vector<Op>& adjoint_program(bool of_forward) const { return adj_[of_forward ? 0 : 1]; }
   void* device_buffer(int id) const { return bufs_.at(id); }
   cudaError_t launch_op(const Op& op, const dev::StageArgs& A, cudaStream_t stream) const {
     return launch_stage(op, A, stream);
@@ -223,6 +225,13 @@ class Plan {
   std::int64_t flex_twiddle(int r1, int r2);
   void select_flex(Op& op) const;
   bool add_flex(Op& op);
+  // line addressing of one side of a stage (see StageArgs)
+  struct LineSide {
+    int affine = 0, atab = 0;
+    std::int64_t base = 0, stride = 1;
+  };
+  bool line_side(int l, std::size_t a, bool afast, bool tables, LineSide* s) const;
+  static void set_lines(dev::StageArgs& A, const LineSide& src, const LineSide& dst);
   std::int64_t add_geo(const Layout& L, const BlockInfo& b, std::size_t pc);
   void build_fused(bool forward);
   void build_literal(bool forward);

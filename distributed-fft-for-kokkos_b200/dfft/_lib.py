@@ -86,6 +86,19 @@ EXCHANGE_FN = ctypes.CFUNCTYPE(ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, 
                                ctypes.c_uint64, ctypes.c_void_p)
 
 
+class StageInfo(ctypes.Structure):
+    _fields_ = [
+        ("kernel", ctypes.c_int32),
+        ("n", ctypes.c_int32),
+        ("two_pass", ctypes.c_int32),
+        ("lines", ctypes.c_int32),
+        ("general", ctypes.c_int32 * 2),
+        ("axis_table", ctypes.c_int32 * 2),
+        ("base", ctypes.c_int64 * 2),
+        ("stride", ctypes.c_int64 * 2),
+    ]
+
+
 class NsDiag(ctypes.Structure):
     _fields_ = [("energy", ctypes.c_double), ("enstrophy", ctypes.c_double), ("divergence_l2", ctypes.c_double)]
 
@@ -141,6 +154,8 @@ SIGNATURES = {
         ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32, ctypes.c_void_p,
                        ctypes.c_uint64]),
     "dfft_get_device_error": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32)]),
+    "dfft_debug_get_stage": (
+        ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.POINTER(StageInfo)]),
     "dfft_get_launch_count": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]),
     "dfft_get_workspace_bytes": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]),
     "dfft_get_all_topologies": (

@@ -20,7 +20,7 @@ import enum
 
 import numpy as np
 
-from ._lib import BlockInfo, PlanDesc, lib, MAX_RANK
+from ._lib import BlockInfo, PlanDesc, StageInfo, lib, MAX_RANK
 
 
 class Direction(enum.IntEnum):
@@ -219,6 +219,17 @@ class Plan:
         _check(lib.dfft_get_topology_chain(self._h, ctypes.byref(n), topos, tr, lay))
         t = [tuple(topos[i * self.rank:(i + 1) * self.rank]) for i in range(cnt)]
         return t, list(tr[:max(cnt - 1, 0)]), list(lay[:cnt])
+
+    def stages(self, program=0):
+        """What each step of a program launches and how it addresses its lines
+        (dfft_debug_get_stage): 0 forward, 1 backward, 2 adjoint of forward, 3
+        adjoint of backward."""
+        out = []
+        while True:
+            info = StageInfo()
+            if lib.dfft_debug_get_stage(self._h, program, len(out), ctypes.byref(info)) != 0:
+                return out
+            out.append(info)
 
     def launch_count(self, direction=Direction.forward):
         n = ctypes.c_int64()

@@ -503,6 +503,35 @@ dfft_status dfft_debug_export_buffers(const dfft_plan* plan, int32_t direction, 
  * No counterpart in the reference. */
 dfft_status dfft_get_device_error(const dfft_plan* plan, int32_t reset, int32_t* code);
 
+/* One step of a plan's programs as it would launch: which kernel, and how that
+ * kernel addresses the lines of its two sides.  `program`: 0 forward, 1
+ * backward, 2 adjoint of forward, 3 adjoint of backward; `step` counts the
+ * kernels of the program from 0.  Host query: plans of dfft_plan_analyze (the
+ * defaults) and executable ones (the tuned choice).  No counterpart in the
+ * reference. */
+enum {
+  DFFT_KERNEL_OTHER = -1,     /* not an FFT stage: copies, transposes, the parts of multi-kernel stages */
+  DFFT_KERNEL_TABLE = 0,      /* table-driven shared-memory stage */
+  DFFT_KERNEL_REGISTER = 1,   /* register stage, one line per thread group */
+  DFFT_KERNEL_PAIR = 2,       /* two complex64 lines per thread */
+  DFFT_KERNEL_PAIR_STREAM = 3, /* the same, several tiles per block */
+  DFFT_KERNEL_PAIR_TMA = 4,
+  DFFT_KERNEL_TWO_PASS = 5,
+  DFFT_KERNEL_TWO_PASS_CHIRP = 6
+};
+typedef struct {
+  int32_t kernel;    /* DFFT_KERNEL_* */
+  int32_t n;         /* line length (real length for R2C / C2R) */
+  int32_t two_pass;  /* 1: the two-pass kernel takes the stage (it is the one, or a choice of the tuner) */
+  int32_t lines;     /* complex lines per tile */
+  /* per side (0 source, 1 destination): 1 = base and stride from the general
+   * tables, the axis table instead of base + position * stride, that base and
+   * stride in elements */
+  int32_t general[2], axis_table[2];
+  int64_t base[2], stride[2];
+} dfft_stage_info;
+dfft_status dfft_debug_get_stage(const dfft_plan* plan, int32_t program, int64_t step, dfft_stage_info* info);
+
 /* Number of kernel launches one dfft_execute issues in a direction. */
 dfft_status dfft_get_launch_count(const dfft_plan* plan, int32_t direction, int64_t* launches);
 
