@@ -175,9 +175,9 @@ int batch_stage_lines(bool dbl, int n);
 cudaError_t launch_fft_batch(BatchParams& P, bool dbl, int kind, bool inverse, bool afast, cudaStream_t st);
 cudaError_t launch_fft_batch_pair(BatchParams& P, bool inverse, bool afast, cudaStream_t st);
 // Two-pass stage of lines of m = R1 R2 points (fft_flex.cuh), or the chirp-z
-// form of it (chirp != null: n-point lines through a convolution of length
-// m >= 2 n - 1); geometry, layouts, tile (A.B complex lines) and scale in the
-// StageArgs.
+// form of it (chirp != null: n-point lines through a convolution of length m,
+// flex_chirp_length; real lines one by one); geometry, layouts, tile (A.B
+// complex lines) and scale in the StageArgs.
 struct FlexArgs {
   int n, m;
   int inverse;         // set by the launcher
@@ -191,7 +191,7 @@ struct FlexArgs {
 bool flex_split(int m, bool chirp, int* R1, int* R2);
 // convolution length of an n-point chirp-z line (0: none long enough)
 int flex_chirp_length(int n);
-// complex lines per tile (two real lines each for R2C / C2R)
+// complex lines per tile (two real lines each for R2C / C2R, chirp-z: one)
 int flex_lines(bool dbl, bool afast, int R1);
 cudaError_t launch_fft_flex(const StageArgs& A, const FlexArgs& F, bool dbl, int kind, bool inverse, cudaStream_t st);
 // Chirp-z (Bluestein) stage for line lengths the radix passes do not cover

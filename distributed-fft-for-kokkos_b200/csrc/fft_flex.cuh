@@ -13,7 +13,7 @@
 // Measured (B200, forward + backward; before: the table-driven kernel of
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
 // kernels): 300 x 250 x 360 complex64 3818 -> 544 us, 200 x 180 x 252 R2C / C2R
-// double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 155 us, 256^3
+// double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 200 us, 256^3
 // complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1131 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
@@ -34,6 +34,11 @@
 //
 // Inverse transforms take the forward codelets' outputs in reverse order,
 // X_{m-k}.
+//
+// R2C / C2R lines go in pairs, one as the real and one as the imaginary part
+// of a complex line, as in the other kernels.  Chirp-z ones go alone: a pair
+// shares its rounding errors and its infinities, and the kernels that longer
+// lines of these lengths take (bluestein.cu) do not pair.
 #pragma once
 
 #include "fft_codelet.cuh"
@@ -191,15 +196,15 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
     fft_flex_kernel(const __grid_constant__ StageArgs A, const __grid_constant__ FlexArgs F) {
   using C = cplx<T>;
   using S = Shape<T, KIND, AFAST, R1, R2, CHIRP>;
-  constexpr bool kReal = KIND == kR2C || KIND == kC2R;
+  constexpr bool kPairs = (KIND == kR2C || KIND == kC2R) && !CHIRP;  // two real lines a complex line
   constexpr int B = S::B, M = S::m;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const s = reinterpret_cast<C*>(smem_raw);
   release_dependents();
   const int t = threadIdx.x;
-  const int per = kReal ? 2 * B : B;
+  const int per = kPairs ? 2 * B : B;
   const int b0 = static_cast<int>(blockIdx.x) * per, nb = min(per, A.Eb - b0);
-  const int nact = kReal ? (nb + 1) / 2 : nb;  // complex lines in the tile
+  const int nact = kPairs ? (nb + 1) / 2 : nb;  // complex lines in the tile
   const int co0 = blockIdx.y, co1 = blockIdx.z;
   const int n = CHIRP ? F.n : M;
   const bool inverse = KIND == kC2R || F.inverse;
@@ -221,53 +226,49 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
   const bool act1 = (AFAST ? t < B * R1 : j1 < R1) && line1 < nact;
 
   dependency_wait();
-  if constexpr (KIND == kC2R && CHIRP) {
-    // Z = X0 + i X1 over the full line, from the two half spectra (imaginary
-    // parts of DC and Nyquist dropped), in natural order
-    constexpr int TPL = S::NT / B;  // threads a line
-    const int line = t / TPL;
-    if (line < nact) {
-      const bool two = 2 * line + 1 < nb;
-      const C* x0 = reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line, co0, co1).base;
-      const C* x1 = two ? reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line + 1, co0, co1).base : x0;
-      const T wt = T(A.weight);
-      for (int k = t % TPL; k <= n / 2; k += TPL) {
-        C c0 = x0[k];
-        C c1 = two ? x1[k] : mk<T>(T(0), T(0));
-        if (k == 0 || 2 * k == n) {
-          at(line, k) = mk<T>(c0.x, c1.x);
-        } else {
-          c0 = cscale(c0, wt);
-          c1 = cscale(c1, wt);
-          at(line, k) = mk<T>(c0.x - c1.y, c0.y + c1.x);
-          at(line, n - k) = mk<T>(c0.x + c1.y, c1.x - c0.y);
-        }
-      }
-    }
-    __syncthreads();
-  }
   // ---- pass 1: codelets over positions j + r R2, row j of the matrix
   C v[R1];
   if (act2) {
-    if constexpr (KIND == kR2C) {
+    if constexpr (CHIRP) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r) v[r] = mk<T>(T(0), T(0));
+      const Line l = src_line(A, b0 + line2, co0, co1);
+      if constexpr (KIND == kR2C) {
+        const T* in = reinterpret_cast<const T*>(A.in);
+        positions<R1, R2, AFAST, true>(l, j2, n, [&](int r, int64_t o) { v[r].x = in[o]; });
+      } else if constexpr (KIND == kC2R) {
+        // the full line from its half spectrum (imaginary parts of DC and
+        // Nyquist dropped), every mode loaded for both positions it makes
+        const C* x = reinterpret_cast<const C*>(A.in) + l.base;
+        const T wt = T(A.weight);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+          const int p = j2 + r * R2;
+          if (p >= n) continue;
+          const int q = 2 * p > n ? n - p : p;
+          const C c = x[q];
+          v[r] = (q == 0 || 2 * q == n) ? mk<T>(c.x, T(0)) : mk<T>(c.x * wt, (q < p ? -c.y : c.y) * wt);
+        }
+      } else {
+        const C* in = reinterpret_cast<const C*>(A.in);
+        positions<R1, R2, AFAST, true>(l, j2, n, [&](int r, int64_t o) { v[r] = in[o]; });
+      }
+#pragma unroll
+      for (int r = 0; r < R1; ++r)
+        if (j2 + r * R2 < n) v[r] = cmul(v[r], chirp(j2 + r * R2));
+    } else if constexpr (KIND == kR2C) {
       const T* in = reinterpret_cast<const T*>(A.in);
 #pragma unroll
       for (int r = 0; r < R1; ++r) v[r] = mk<T>(T(0), T(0));
-      positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + 2 * line2, co0, co1), j2, n,
+      positions<R1, R2, AFAST, false>(src_line(A, b0 + 2 * line2, co0, co1), j2, 0,
                                       [&](int r, int64_t o) { v[r].x = in[o]; });
       if (2 * line2 + 1 < nb)
-        positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + 2 * line2 + 1, co0, co1), j2, n,
+        positions<R1, R2, AFAST, false>(src_line(A, b0 + 2 * line2 + 1, co0, co1), j2, 0,
                                         [&](int r, int64_t o) { v[r].y = in[o]; });
-    } else if constexpr (KIND == kC2R && CHIRP) {
-#pragma unroll
-      for (int r = 0; r < R1; ++r)
-        v[r] = j2 + r * R2 < n ? at(line2, j2 + r * R2) : mk<T>(T(0), T(0));
     } else if constexpr (KIND == kC2R) {
       // Z from the half spectra directly, every mode loaded for both positions
-      // it makes: through shared memory as in the chirp-z form, with its
-      // barriers, 384^3 double took 273 us where this form took 221 (131 x 105 x 157
-      // chirp-z lines, where the loads' index choices weigh more, 36 instead of
-      // 46)
+      // it makes: assembled in shared memory, with the barriers that takes,
+      // 384^3 double took 273 us where this form took 221
       const bool two = 2 * line2 + 1 < nb;
       const C* x0 = reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2, co0, co1).base;
       const C* x1 = two ? reinterpret_cast<const C*>(A.in) + src_line(A, b0 + 2 * line2 + 1, co0, co1).base : x0;
@@ -289,22 +290,10 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
       }
     } else {
       const C* in = reinterpret_cast<const C*>(A.in);
-      if (CHIRP) {
-#pragma unroll
-        for (int r = 0; r < R1; ++r) v[r] = mk<T>(T(0), T(0));
-      }
-      positions<R1, R2, AFAST, CHIRP>(src_line(A, b0 + line2, co0, co1), j2, n,
+      positions<R1, R2, AFAST, false>(src_line(A, b0 + line2, co0, co1), j2, 0,
                                       [&](int r, int64_t o) { v[r] = in[o]; });
     }
-    if (CHIRP) {
-#pragma unroll
-      for (int r = 0; r < R1; ++r)
-        if (j2 + r * R2 < n) v[r] = cmul(v[r], chirp(j2 + r * R2));
-    }
     Dft<T, R1>::run(v);
-  }
-  if constexpr (KIND == kC2R && CHIRP) __syncthreads();  // every position read: the buffer takes the matrices
-  if (act2) {
     C* o = &at(line2, j2 * row1);
 #pragma unroll
     for (int r = 0; r < R1; ++r) o[r * el] = v[r];
@@ -383,32 +372,26 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
         x[r] = w[(R1 - r) % R1];
         if (j2 + r * R2 < n) x[r] = cmul(x[r], chirp(j2 + r * R2));
       }
+      const Line l = dst_line(A, b0 + line2, co0, co1);
       if constexpr (KIND == kC2C) {
         C* out = reinterpret_cast<C*>(A.out);
-        positions<R1, R2, AFAST, true>(dst_line(A, b0 + line2, co0, co1), j2, n,
-                                       [&](int r, int64_t o) { out[o] = cscale(x[r], scale); });
+        positions<R1, R2, AFAST, true>(l, j2, n, [&](int r, int64_t o) { out[o] = cscale(x[r], scale); });
       } else if constexpr (KIND == kC2R) {
         T* out = reinterpret_cast<T*>(A.out);
-        positions<R1, R2, AFAST, true>(dst_line(A, b0 + 2 * line2, co0, co1), j2, n,
-                                       [&](int r, int64_t o) { out[o] = x[r].x * scale; });
-        if (2 * line2 + 1 < nb)
-          positions<R1, R2, AFAST, true>(dst_line(A, b0 + 2 * line2 + 1, co0, co1), j2, n,
-                                         [&](int r, int64_t o) { out[o] = x[r].y * scale; });
+        positions<R1, R2, AFAST, true>(l, j2, n, [&](int r, int64_t o) { out[o] = x[r].x * scale; });
       } else {
-#pragma unroll
-        for (int r = 0; r < R1; ++r) w[r] = x[r];
+        C* out = reinterpret_cast<C*>(A.out);
+        const T sw = scale * T(A.weight);
+        positions<R1, R2, AFAST, true>(l, j2, n / 2 + 1, [&](int r, int64_t o) {
+          const int k = j2 + r * R2;
+          out[o] = (k == 0 || 2 * k == n) ? mk<T>(x[r].x * scale, T(0)) : cscale(x[r], sw);
+        });
       }
     }
-    if constexpr (KIND != kR2C) return;
-    __syncthreads();
-    if (act2) {
-#pragma unroll
-      for (int r = 0; r < R1; ++r)
-        if (j2 + r * R2 < n) at(line2, j2 + r * R2) = w[r];
-    }
+    return;
   }
   // ---- R2C: the two half spectra of a line pair from its full spectrum
-  if constexpr (KIND == kR2C) {
+  if constexpr (KIND == kR2C && !CHIRP) {
     __syncthreads();
     constexpr int TPL = S::NT / B;  // threads a line
     const int line = t / TPL;
@@ -418,10 +401,10 @@ __global__ void __launch_bounds__((Shape<T, KIND, AFAST, R1, R2, CHIRP>::NT),
       const bool two = 2 * line + 1 < nb;
       C* y0 = out + dst_line(A, b0 + 2 * line, co0, co1).base;
       C* y1 = two ? out + dst_line(A, b0 + 2 * line + 1, co0, co1).base : y0;
-      for (int k = t % TPL; k <= n / 2; k += TPL) {
+      for (int k = t % TPL; k <= M / 2; k += TPL) {
         const C a = at(line, k);
-        const C b = cconj(at(line, k == 0 ? 0 : n - k));
-        const T hs = (k == 0 || 2 * k == n) ? h0 : h1;
+        const C b = cconj(at(line, k == 0 ? 0 : M - k));
+        const T hs = (k == 0 || 2 * k == M) ? h0 : h1;
         y0[k] = cscale(cadd(a, b), hs);
         if (two) {
           const C d = csub(a, b);

@@ -412,7 +412,7 @@ void Plan::select_flex(Op& op) const {
   dev::StageArgs& A = op.sa;
   A.pairs = 4;
   A.B = op.flex_B;
-  const int per = op.kind == dev::kC2C ? A.B : 2 * A.B;
+  const int per = op.kind == dev::kC2C || op.chirp ? A.B : 2 * A.B;
   A.tiles_b = (A.Eb + per - 1) / per;
   op.tiles = static_cast<unsigned>(static_cast<unsigned long long>(A.tiles_b) * A.Eo0 * A.Eo1);
 }
@@ -487,7 +487,7 @@ bool Plan::add_flex(Op& op) {
   const bool chirp = !radix_supported(static_cast<std::size_t>(A.n));
   const int m = chirp ? dev::flex_chirp_length(A.n) : A.n;
   if (m == 0 || !dev::flex_split(m, chirp, &r1, &r2)) return false;
-  const int B = dev::flex_lines(d_.dbl, afast, r1), per = real ? 2 * B : B;
+  const int B = dev::flex_lines(d_.dbl, afast, r1), per = real && !chirp ? 2 * B : B;
   if (static_cast<unsigned long long>((A.Eb + per - 1) / per) * A.Eo0 * A.Eo1 >= (1ull << 31)) return false;
   op.flex = true;
   op.flex_B = B;
