@@ -13,7 +13,7 @@
 // Measured (B200, forward + backward; before: the table-driven kernel of
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
 // kernels): 300 x 250 x 360 complex64 3818 -> 544 us, 200 x 180 x 252 R2C / C2R
-// double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 200 us, 256^3
+// double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 190 us, 256^3
 // complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1131 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
