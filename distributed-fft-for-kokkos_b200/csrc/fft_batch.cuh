@@ -106,21 +106,21 @@ size_t tile_smem(int n, bool afast) {
   }
 }
 
-template <int THREADS, typename K>
+template <typename C, int THREADS, typename K>
 cudaError_t launch_tiles(K kernel, const BatchParams& P, size_t smem, cudaStream_t st) {
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) return e;
   const long long total = P.prefix[P.nfields];
   if (total < 1) return cudaSuccess;
   if (total >= (1ll << 31)) return cudaErrorInvalidConfiguration;
-  return launch_kernel_early(true, kernel, dim3(static_cast<unsigned>(total)), THREADS, smem, st, P);
+  return launch_kernel_early(early_start(P, sizeof(C)), kernel, dim3(static_cast<unsigned>(total)), THREADS, smem, st, P);
 }
 
 template <bool INV, bool AFAST, int N>
 cudaError_t launch_batch_pair_n(BatchParams& P, cudaStream_t st) {
   constexpr size_t smem = pair_tile_smem<N, BatchPairs<N, AFAST>::value, AFAST>();
   for (int i = 0; i < P.nfields; ++i) P.f[i] = with_table_offsets(P.f[i]);
-  return launch_tiles<BatchPairs<N, AFAST>::threads>(fft_batch_pair_kernel<INV, AFAST, N>, P, smem, st);
+  return launch_tiles<float2, BatchPairs<N, AFAST>::threads>(fft_batch_pair_kernel<INV, AFAST, N>, P, smem, st);
 }
 
 template <typename T, bool AFF, int N>
@@ -128,13 +128,13 @@ cudaError_t launch_batch_n(BatchParams& P, size_t smem, int kind, bool inverse, 
   constexpr int NT = BatchLines<T, N>::threads;
   if (kind == kC2C) {
     if (inverse)
-      return afast ? launch_tiles<NT>(fft_batch_c2c_kernel<T, true, true, AFF, N>, P, smem, st)
-                   : launch_tiles<NT>(fft_batch_c2c_kernel<T, true, false, AFF, N>, P, smem, st);
-    return afast ? launch_tiles<NT>(fft_batch_c2c_kernel<T, false, true, AFF, N>, P, smem, st)
-                 : launch_tiles<NT>(fft_batch_c2c_kernel<T, false, false, AFF, N>, P, smem, st);
+      return afast ? launch_tiles<cplx<T>, NT>(fft_batch_c2c_kernel<T, true, true, AFF, N>, P, smem, st)
+                   : launch_tiles<cplx<T>, NT>(fft_batch_c2c_kernel<T, true, false, AFF, N>, P, smem, st);
+    return afast ? launch_tiles<cplx<T>, NT>(fft_batch_c2c_kernel<T, false, true, AFF, N>, P, smem, st)
+                 : launch_tiles<cplx<T>, NT>(fft_batch_c2c_kernel<T, false, false, AFF, N>, P, smem, st);
   }
-  if (kind == kR2C) return launch_tiles<NT>(fft_batch_real_kernel<T, false, AFF, N>, P, smem, st);
-  if (kind == kC2R) return launch_tiles<NT>(fft_batch_real_kernel<T, true, AFF, N>, P, smem, st);
+  if (kind == kR2C) return launch_tiles<cplx<T>, NT>(fft_batch_real_kernel<T, false, AFF, N>, P, smem, st);
+  if (kind == kC2R) return launch_tiles<cplx<T>, NT>(fft_batch_real_kernel<T, true, AFF, N>, P, smem, st);
   return cudaErrorInvalidValue;
 }
 

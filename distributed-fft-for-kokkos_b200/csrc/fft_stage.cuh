@@ -121,9 +121,19 @@ inline cudaError_t launch_kernel_early(bool early, void (*kernel)(P...), dim3 gr
   return e;
 }
 
-// a stage's early start: by the bytes of the array it reads (complex elements)
+// a launch's early start: by the bytes of the arrays it reads (complex elements)
+inline size_t stage_bytes(const StageArgs& A, size_t elem) { return static_cast<size_t>(A.n) * A.Eb * A.Eo0 * A.Eo1 * elem; }
 inline bool early_start(const StageArgs& A, size_t elem) {
-  return !A.plain_launch && static_cast<size_t>(A.n) * A.Eb * A.Eo0 * A.Eo1 * elem <= kEarlyStartBytes;
+  return !A.plain_launch && stage_bytes(A, elem) <= kEarlyStartBytes;
+}
+inline bool early_start(const BatchParams& P, size_t elem) {
+  size_t bytes = 0;
+  bool plain = false;
+  for (int i = 0; i < P.nfields; ++i) {
+    bytes += stage_bytes(P.f[i], elem);
+    plain = plain || P.f[i].plain_launch;
+  }
+  return !plain && bytes <= kEarlyStartBytes;
 }
 
 // Element offset of global coordinate c (nd axes) in a layout.
