@@ -124,6 +124,31 @@ void Batch::launch_group(const Group& g, cudaStream_t st) const {
   }
 }
 
+// whether the output of a field overlaps the input or output of a field of
+// another group
+bool Batch::shares_memory(const void* const* ins, void* const* outs, bool forward,
+                          const std::vector<int>& group) const {
+  struct Range {
+    std::uintptr_t begin, end;
+    int group;
+    bool written;
+  };
+  std::vector<Range> r;
+  for (std::size_t f = 0; f < plans_.size(); ++f) {
+    const PlanDesc& d = plans_[f]->desc();
+    const std::size_t real = dbl_ ? 8 : 4;
+    const std::size_t in = total_size(d.gin) * real * (d.r2c ? 1 : 2), out = total_size(d.gout) * real * 2;
+    const auto a = reinterpret_cast<std::uintptr_t>(ins[f]), b = reinterpret_cast<std::uintptr_t>(outs[f]);
+    r.push_back(Range{a, a + (forward ? in : out), group[f], false});
+    r.push_back(Range{b, b + (forward ? out : in), group[f], true});
+  }
+  std::sort(r.begin(), r.end(), [](const Range& x, const Range& y) { return x.begin < y.begin; });
+  for (std::size_t i = 0; i < r.size(); ++i)
+    for (std::size_t j = i + 1; j < r.size() && r[j].begin < r[i].end; ++j)
+      if (r[i].group != r[j].group && (r[i].written || r[j].written)) return true;
+  return false;
+}
+
 void Batch::execute(const void* const* ins, void* const* outs, bool forward, cudaStream_t st) const {
   if (!ins || !outs) fail(kErrInvalidArgument, "null buffer arrays");
   for (std::size_t f = 0; f < plans_.size(); ++f) plans_[f]->check_buffers(ins[f], outs[f], forward);
@@ -172,13 +197,16 @@ void Batch::execute(const void* const* ins, void* const* outs, bool forward, cud
     }
   }
   // Fields that share a launch at one stage share it at every stage (cubic
-  // fields): each group's stages follow one another on a lane of their own,
-  // without waiting for the other groups between stages.  Else the groups of
-  // one stage run concurrently and join before the next.
+  // fields), and none writes to memory that a field of another group uses: each
+  // group's stages follow one another on a lane of their own, without waiting
+  // for the other groups between stages.  Else the groups of one stage run
+  // concurrently and join before the next, so that every input has been read
+  // before the last stages write.
   bool chains = true;
   for (std::size_t s = 0; s < nst; ++s)
     chains = chains && single[s].empty() && member[s] == member[0];
-  if (chains && nst > 0) {
+  chains = chains && nst > 0 && !shares_memory(ins, outs, forward, member[0]);
+  if (chains) {
     const int nl = static_cast<int>(groups[0].size());
     fork(st, nl);
     for (std::size_t s = 0; s < nst; ++s)

@@ -45,6 +45,7 @@ class Batch {
     std::vector<dev::StageArgs> args;
   };
   void launch_group(const Group& g, cudaStream_t st) const;
+  bool shares_memory(const void* const* ins, void* const* outs, bool forward, const std::vector<int>& group) const;
   std::vector<const Plan*> plans_;
   bool dbl_ = false;
   cudaStream_t aux_[kAux] = {};
