@@ -181,7 +181,7 @@ cudaError_t launch_fft_batch_pair(BatchParams& P, bool inverse, bool afast, cuda
 struct FlexArgs {
   int n, m;
   int inverse;         // set by the launcher
-  const void* tw;      // [a < R2][b < R1] w_m^(a b), then [a < R1][b < R2]
+  const void* tw;      // [a < R2][b < R1] w_m^(a b), chirp-z: then [a < R1][b < R2]
   const void* chirp;   // chirp-z: n values exp(-i pi (j^2 mod 2n) / n)
   const void* filter;  // chirp-z: m values (see BlueArgs), forward and inverse
   const void* filter_inverse;

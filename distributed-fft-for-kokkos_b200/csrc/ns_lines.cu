@@ -216,8 +216,8 @@ class Lines final : public NsLines {
     x_ = dmalloc(9 * xq());
     y_ = dmalloc(9 * xyz());
     for (auto ax : {std::make_pair(&g_.x, ex_), std::make_pair(&g_.y, ey_), std::make_pair(&g_.z, ez_)}) {
-      const std::vector<double> h = two_pass_twiddles(ax.second->R1, ax.second->R2);
-      const std::vector<T> t(h.begin(), h.begin() + 2 * ax.first->n);
+      const std::vector<double> h = two_pass_twiddles(ax.second->R1, ax.second->R2, false);
+      const std::vector<T> t(h.begin(), h.end());
       C* p = dmalloc(static_cast<std::size_t>(ax.first->n));
       ck(cudaMemcpy(p, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice), "ns twiddles");
       ax.first->tw = p;

@@ -123,32 +123,61 @@ void host_fft(std::vector<long double>& re, std::vector<long double>& im) {
   }
 }
 
-// FFT of m long double values: radix 2 for powers of two, else the plain sum
-// over the m-th roots of unity (m is at most a few hundred points there).
+// exp(-2 pi i k / m), k < m
+struct Roots {
+  std::vector<long double> c, s;
+  explicit Roots(std::size_t m) : c(m), s(m) {
+    const long double pi = 3.141592653589793238462643383279502884L;
+    for (std::size_t k = 0; 2 * k <= m; ++k) {
+      const long double ang = -2.0L * pi * static_cast<long double>(k) / static_cast<long double>(m);
+      c[k] = cosl(ang);
+      s[k] = sinl(ang);
+      if (k > 0) {
+        c[m - k] = c[k];
+        s[m - k] = -s[k];
+      }
+    }
+    if (m % 2 == 0) s[m / 2] = 0.0L;
+  }
+};
+
+// DFT of the n values at x + stride * j into y, w the n * stride-th roots:
+// the p interleaved parts of n / p values, p the smallest prime factor, then
+// p-point sums, so m (p1 + p2 + ...) products in all.
+void host_dft_part(const long double* xr, const long double* xi, std::size_t stride, std::size_t n, const Roots& w,
+                   long double* yr, long double* yi) {
+  if (n == 1) {
+    yr[0] = xr[0];
+    yi[0] = xi[0];
+    return;
+  }
+  std::size_t p = 2;
+  while (n % p != 0) ++p;
+  const std::size_t q = n / p;
+  std::vector<long double> tr(n), ti(n);
+  for (std::size_t r = 0; r < p; ++r)
+    host_dft_part(xr + r * stride, xi + r * stride, stride * p, q, w, tr.data() + r * q, ti.data() + r * q);
+  for (std::size_t k = 0; k < n; ++k) {
+    long double ar = 0.0L, ai = 0.0L;
+    for (std::size_t r = 0; r < p; ++r) {
+      const std::size_t e = (r * k) % n * stride, t = r * q + k % q;
+      ar += tr[t] * w.c[e] - ti[t] * w.s[e];
+      ai += tr[t] * w.s[e] + ti[t] * w.c[e];
+    }
+    yr[k] = ar;
+    yi[k] = ai;
+  }
+}
+
+// FFT of m long double values: radix 2 for powers of two, else by factors
 void host_dft(std::vector<long double>& re, std::vector<long double>& im) {
   const std::size_t m = re.size();
   if ((m & (m - 1)) == 0) {
     host_fft(re, im);
     return;
   }
-  const long double pi = 3.141592653589793238462643383279502884L;
-  std::vector<long double> c(m), s(m), xr(re), xi(im);
-  for (std::size_t k = 0; k < m; ++k) {
-    const long double ang = -2.0L * pi * static_cast<long double>(k) / static_cast<long double>(m);
-    c[k] = cosl(ang);
-    s[k] = sinl(ang);
-  }
-  for (std::size_t k = 0; k < m; ++k) {
-    long double ar = 0.0L, ai = 0.0L;
-    for (std::size_t j = 0, e = 0; j < m; ++j) {
-      ar += xr[j] * c[e] - xi[j] * s[e];
-      ai += xr[j] * s[e] + xi[j] * c[e];
-      e += k;
-      if (e >= m) e -= m;
-    }
-    re[k] = ar;
-    im[k] = ai;
-  }
+  const std::vector<long double> xr(re), xi(im);
+  host_dft_part(xr.data(), xi.data(), 1, m, Roots(m), re.data(), im.data());
 }
 
 }  // namespace
@@ -372,31 +401,31 @@ const void* Plan::twiddle(std::size_t n) {
 }
 
 // Twiddles of an m = r1 r2 point two-pass transform, w_m = exp(-2 pi i / m):
-// [a < r2][b < r1] w_m^(a b), then [a < r1][b < r2] (re, im interleaved).
-std::vector<double> two_pass_twiddles(int r1, int r2) {
-  const int m = r1 * r2;
-  const long double pi = 3.141592653589793238462643383279502884L;
+// [a < r2][b < r1] w_m^(a b), then, for the way back of a chirp-z line, [a <
+// r1][b < r2] (re, im interleaved).
+std::vector<double> two_pass_twiddles(int r1, int r2, bool back) {
+  const Roots w(static_cast<std::size_t>(r1) * r2);
   std::vector<double> h;
-  h.reserve(4 * static_cast<std::size_t>(m));
-  auto put = [&](int a, int b) {
-    const long double ang = 2.0L * pi * static_cast<long double>(a * b) / static_cast<long double>(m);
-    h.push_back(static_cast<double>(cosl(ang)));
-    h.push_back(static_cast<double>(-sinl(ang)));
+  h.reserve((back ? 4 : 2) * w.c.size());
+  auto put = [&](int rows, int columns) {
+    for (int a = 0; a < rows; ++a)
+      for (int b = 0; b < columns; ++b) {
+        h.push_back(static_cast<double>(w.c[static_cast<std::size_t>(a) * b]));
+        h.push_back(static_cast<double>(w.s[static_cast<std::size_t>(a) * b]));
+      }
   };
-  for (int a = 0; a < r2; ++a)
-    for (int b = 0; b < r1; ++b) put(a, b);
-  for (int a = 0; a < r1; ++a)
-    for (int b = 0; b < r2; ++b) put(a, b);
+  put(r2, r1);
+  if (back) put(r1, r2);
   return h;
 }
 
 // The table in the plan's precision, stored with the layout tables (one
 // upload): its offset there.
-std::int64_t Plan::flex_twiddle(int r1, int r2) {
-  auto key = std::make_pair(r1, r2);
+std::int64_t Plan::flex_twiddle(int r1, int r2, bool back) {
+  auto key = std::make_tuple(r1, r2, back);
   auto it = flex_tables_.find(key);
   if (it != flex_tables_.end()) return it->second;
-  const std::vector<double> h = two_pass_twiddles(r1, r2);
+  const std::vector<double> h = two_pass_twiddles(r1, r2, back);
   const std::vector<float> hf(h.begin(), h.end());
   const std::size_t bytes = h.size() * (d_.dbl ? 8 : 4);
   if (host_tables_.size() % 2) host_tables_.push_back(0);  // 16-byte elements
@@ -494,7 +523,7 @@ bool Plan::add_flex(Op& op) {
   op.fx = dev::FlexArgs{};
   op.fx.n = A.n;
   op.fx.m = m;
-  op.fx_tw = flex_twiddle(r1, r2);  // resolved by allocate_device
+  op.fx_tw = flex_twiddle(r1, r2, chirp);  // resolved by allocate_device
   if (chirp)
     bluestein_tables(static_cast<std::size_t>(A.n), static_cast<std::size_t>(m), &op.fx.chirp, &op.fx.filter,
                      &op.fx.filter_inverse);

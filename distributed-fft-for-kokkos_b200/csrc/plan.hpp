@@ -8,6 +8,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "dev_types.h"
@@ -69,7 +70,7 @@ struct TmaSource {
 bool tma_encode(void* map, const void* base, const TmaSource& t);
 
 // Twiddle tables of a two-pass transform (dev::FlexArgs::tw), re / im interleaved.
-std::vector<double> two_pass_twiddles(int r1, int r2);
+std::vector<double> two_pass_twiddles(int r1, int r2, bool back);
 
 struct Op {
   enum Type { Stage, Pack, All2All, Unpack, Scale, Copy, BluePre, BlueMul, BluePost, FourTwiddle } type;
@@ -221,8 +222,8 @@ class Plan {
   std::map<std::pair<std::size_t, std::size_t>, std::vector<void*>> blue_tables_;  // (n, m) -> chirp, filter fwd / inv
   void bluestein_tables(std::size_t n, std::size_t m, const void** chirp, const void** ffwd, const void** finv);
   // Twiddles of an m = R1 R2 point two-pass stage (dev::FlexArgs::tw).
-  std::map<std::pair<int, int>, std::int64_t> flex_tables_;
-  std::int64_t flex_twiddle(int r1, int r2);
+  std::map<std::tuple<int, int, bool>, std::int64_t> flex_tables_;
+  std::int64_t flex_twiddle(int r1, int r2, bool back);
   void select_flex(Op& op) const;
   bool add_flex(Op& op);
   // line addressing of one side of a stage (see StageArgs)
