@@ -6,7 +6,7 @@ import pytest
 
 import dfft
 
-REGISTER, PAIR, PAIR_STREAM, PAIR_TMA = 1, 2, 3, 4  # DFFT_KERNEL_*
+OTHER, REGISTER, PAIR, PAIR_STREAM, PAIR_TMA, TWO_PASS_CHIRP = -1, 1, 2, 3, 4, 6  # DFFT_KERNEL_*
 
 
 def _plan(gin, **kw):
@@ -45,3 +45,14 @@ def test_two_pass_choice_leaves_the_addressing():
     for program in range(4):
         for s in p.stages(program):
             assert s.two_pass and s.kernel == REGISTER and not s.axis_table[0] and not s.axis_table[1]
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+@pytest.mark.parametrize("first,one_kernel", [(1, False), (2, False), (5, True), (8, True)])
+def test_chirp_rows_across_a_short_axis(first, one_kernel, precision):
+    """One chirp-z kernel only where its tiles (8 lines, 16 with short complex64 codelets) hold more than a quarter."""
+    gin = (first, 16, 251, 32)
+    p = dfft.Plan(gin, gin, (3, 2, 1), (1, 2, 1, 1), (1, 1, 1, 2), layout="left", precision=precision, analyze_only=True)
+    for program in range(4):
+        kernels = [s.kernel for s in p.stages(program)]
+        assert (TWO_PASS_CHIRP in kernels) == one_kernel and (OTHER in kernels) != one_kernel
