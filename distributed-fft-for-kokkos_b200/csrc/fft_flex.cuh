@@ -1,7 +1,8 @@
 // Two-pass FFT stage for lines of m = R1 R2 points, R1 >= R2 two codelet
 // lengths up to 32 (sm_100a): the 2^a 3^b 5^c 7^d lengths up to 512 that split
-// so (and some up to 1024, and short multiples of 11 and 13), and, through the
-// chirp-z convolution, every other length n whose 2 n - 1 fits such an m.
+// so (and some up to 1024, and multiples of 11 and 13 up to 198), and, through
+// the chirp-z convolution, every length n with a larger prime factor and
+// 2 n - 1 <= 1024.
 //
 // What bounds it: bytes.  A tile of B lines is read from global memory once
 // and written once; between the two passes a line crosses shared memory once
@@ -12,9 +13,9 @@
 //
 // Measured (B200, forward + backward; before: the table-driven kernel of
 // fft_stage.cu, five launches per chirp-z stage, the 24- and 8-value register
-// kernels): 300 x 250 x 360 complex64 3818 -> 544 us, 200 x 180 x 252 R2C / C2R
+// kernels): 300 x 250 x 360 complex64 3818 -> 536 us, 200 x 180 x 252 R2C / C2R
 // double 1633 -> 207 us, 131 x 105 x 157 R2C / C2R double 766 -> 190 us, 256^3
-// complex128 644 -> 545 us, 384^3 R2C / C2R double 1568 -> 1131 us.  On 2^k and
+// complex128 644 -> 552 us, 384^3 R2C / C2R double 1568 -> 1124 us.  On 2^k and
 // 3 2^k lines the tuner chooses between this kernel and the older ones, which
 // stay ahead on complex64 (two lines per thread) and short stages.
 //

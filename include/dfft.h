@@ -142,7 +142,11 @@ dfft_status dfft_plan_destroy(dfft_plan* plan);
  * and writes the input layout to `out`.  `in` is not modified.  Asynchronous
  * on the plan's stream.  Each buffer must be aligned to its element type
  * (real or complex of the plan's precision); a misaligned pointer is rejected
- * with DFFT_ERROR_INVALID_ARGUMENT before any launch. */
+ * with DFFT_ERROR_INVALID_ARGUMENT before any launch.
+ * R2C / C2R lines are transformed in pairs of neighbours, so a line's rounding
+ * errors are relative to the larger of the two and an infinity or NaN reaches
+ * both; lines whose length has a prime factor above 13, or is too long for one
+ * stage, are transformed one by one. */
 dfft_status dfft_execute(const dfft_plan* plan, const void* in, void* out, int32_t direction);
 
 /* Same as dfft_execute with an explicit stream (overrides the plan's). */
@@ -279,7 +283,8 @@ dfft_status dfft_graph_destroy(dfft_graph* graph);
  * row orientation (a work table of every field's tiles, any supported line
  * lengths: 2^k up to 2048 and 3 * 2^k up to 768, register kernels), instead
  * of one launch per field; stages outside that set launch per field.  Buffers
- * follow dfft_execute.  Capture dfft_batch_execute in a CUDA graph to replay
+ * follow dfft_execute; an output may lie where another field's input is (fields
+ * of two stages or more: every input is read before any output is written).  Capture dfft_batch_execute in a CUDA graph to replay
  * it.  No counterpart in the reference (its batched Navier-Stokes example
  * drives one plan over 4D views per field,
  * examples/navier-stokes-MPI-batched/main.cpp:465-468). */
